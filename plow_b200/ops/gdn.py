@@ -16,8 +16,11 @@ def gdn(qkvz, ba, conv_w, a_log, dt_bias, conv_state, ssm_state, pos, seq, hk, h
     rows = qkvz.shape[0]
     if out is None:
         out = torch.empty(rows, hv * head_dim, dtype=BF16, device=qkvz.device)
+    # f32 scratch of the two kernels (layout: csrc/cuda/gdn.cu): per row 256 per key head, 128 per v head, gates and dots
+    n = native.cuda_lib().plow_gdn_scratch_bytes(rows, hk, hv)
+    scratch = torch.empty(max(int(n), 16), dtype=torch.uint8, device=qkvz.device)
     native.call("plow_gdn", out, conv_state, ssm_state, qkvz, qkvz.stride(0), ba, ba.stride(0), conv_w, a_log, dt_bias,
-                pos, seq, rows, hk, hv, head_dim, conv)
+                pos, seq, rows, hk, hv, head_dim, conv, scratch)
     return out
 
 

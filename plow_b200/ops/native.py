@@ -57,6 +57,8 @@ def cuda_lib() -> C.CDLL:
     lib = C.CDLL(str(_ensure_built("libplow_cuda.so")), mode=C.RTLD_GLOBAL)
     lib.plow_gemm.argtypes = [C.POINTER(GemmDesc), C.c_void_p]
     lib.plow_gemm.restype = C.c_int
+    lib.plow_gdn_scratch_bytes.argtypes = [C.c_int32] * 3
+    lib.plow_gdn_scratch_bytes.restype = C.c_int64
     return lib
 
 
@@ -143,7 +145,7 @@ _SIGS = {
     "plow_dsa_k_write": "pppipppppp" "iiiifp",
     "plow_dsa_select": "ppippp" "ipipplp" "pppiiiiiipp",
     "plow_dsa_gather": "pppppi" "pppppi" "iip",
-    "plow_gdn": "ppppipi" "ppppp" "iiiiip",
+    "plow_gdn": "ppppipi" "ppppp" "iiiiipp",
     "plow_gated_norm": "pppiipiiifp",
     "plow_sigmoid_gate": "ppplp",
     "plow_gqa_attention": "ppplpipp" "iiiiiii" "pi" "ppppp" "fppp",
@@ -189,7 +191,7 @@ def profile_summary() -> list:
         e[1] += a.elapsed_time(b)
     PROFILE.clear()
     return sorted(((k, c, t) for k, (c, t) in agg.items()), key=lambda x: -x[2])
-_KERNELS_PER_CALL = {"plow_gqa_attention": 2, "plow_dsa_select": 3, "plow_mla_prefill_attention": 3}
+_KERNELS_PER_CALL = {"plow_gqa_attention": 2, "plow_dsa_select": 3, "plow_mla_prefill_attention": 3, "plow_gdn": 2}
 
 
 def call(name: str, *args) -> None:
