@@ -34,7 +34,7 @@ def _case(lens, starts, hk, hv, idle, pad, seed):
 @pytest.mark.parametrize("lens,starts,hk,hv,idle,pad", [
     ([1], [0], 2, 4, 0, 0), ([1, 1, 1], [0, 5, 9], 16, 32, 1, 0), ([2, 3, 4], [0, 7, 0], 2, 2, 0, 0),
     ([7, 8, 9, 1, 2], [0, 11, 0, 3, 1], 2, 4, 2, 1), ([15, 16, 17, 18], [4, 0, 1, 2], 1, 4, 0, 3),
-    ([100, 1, 301], [0, 64, 1000], 2, 4, 1, 2), ([25, 24, 23, 1, 1, 1, 200], [0, 1, 2, 3, 4, 5, 6], 2, 4, 0, 4)])
+    ([100, 1, 301], [0, 64, 1000], 2, 4, 1, 2), ([70, 5, 4, 3, 66], [0, 1, 0, 9, 2], 2, 4, 1, 0), ([25, 24, 23, 1, 1, 1, 200], [0, 1, 2, 3, 4, 5, 6], 2, 4, 0, 4)])
 def test_gdn_runs(lens, starts, hk, hv, idle, pad):
     from plow_b200.ops import gdn
     qkvz, ba, conv_w, a_log, dt_bias, cs, ss, pos, seq, spans = _case(lens, starts, hk, hv, idle, pad, sum(lens))
@@ -52,3 +52,18 @@ def test_gdn_runs(lens, starts, hk, hv, idle, pad):
         assert (ss[i] - S).norm() <= 5e-6 * S.norm(), i
         assert torch.equal(cs[i], h), i
     assert (out[pos < 0] == 7.0).all()
+
+
+@pytest.mark.parametrize("hd,pad,ofs", [(128, 0, 256), (128, 1, 256), (128, 0, 258), (64, 0, 128)])
+def test_gated_norm_layouts(hd, pad, ofs):
+    from plow_b200.ops import gdn
+    rows, heads = 37, 3
+    o = torch.randn(rows, heads * hd, device="cuda").bfloat16()
+    z = torch.randn(rows, ofs + heads * hd + 4 + pad, device="cuda").bfloat16()
+    gamma = torch.rand(hd, device="cuda") + 0.5
+    got = gdn.gated_norm(o, z, ofs, gamma, heads, hd, 1e-6).float().view(rows, heads, hd)
+    x = o.double().view(rows, heads, hd)
+    zz = z[:, ofs:ofs + heads * hd].double().view(rows, heads, hd)
+    want = x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + 1e-6) * gamma.double() * torch.nn.functional.silu(zz)
+    # one rounding to bf16
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()
