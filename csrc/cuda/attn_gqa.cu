@@ -34,6 +34,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
+#include "attn_prefill.h"
 #include "ptx.cuh"
 #include "tmap.cuh"
 
@@ -43,6 +44,10 @@ constexpr int kGqaPage = 64;
 constexpr int kGqaThreads = 192;   // TMA warp, MMA warp, 4 softmax warps
 constexpr int kGqaThreads8 = 320;  // + 4 converter warps (e4m3 cache)
 constexpr int kGqaRaw = 3;         // raw e4m3 tiles in flight; 4 operand stages behind them
+
+// Rows from which an unsplit bf16 call takes the two-tile kernel of attn_prefill.cu: its items are up to twice as long, so
+// it wants many rows; decode steps (one row per sequence) lie below.
+constexpr int kPrefillRows = 256;
 
 struct GqaItem { int r0, nt, kvh, split, tile0, ntiles, slot, ns; };
 
@@ -57,15 +62,10 @@ struct GqaArgs {
   int* status;
   int rows, nq, nkv, group, max_pages, max_splits, window;
   float scale_log2e;
-  // materialised multi-head latent attention: the last `kr_slabs` key slabs come from a separate tensor shared by
-  // all heads (the rotary part), and the value tile sits `v_x0` columns into the key tensor's head block
-  int kr_slabs, v_x0;
-  int head_major;          // items are [chunk][head] (one split): visit them head by head
   const float* kv_scale;   // e4m3 cache: [n_pages][64][2 * nkv] f32, k scales then v scales of a token
 };
 
-// HDQ = width of a query / key row, HDV = width of a value row.  They differ for multi-head latent attention in its
-// materialised form (192 = 128 no-position + 64 rotary dims against 128 value dims).
+// HDQ = width of a query / key row, HDV = width of a value row.
 template <int HDQ, int HDV, bool KV8 = false> struct GqaCfg {
   static constexpr int kSlabsQ = HDQ / 64;               // 64-column (128-byte) slabs per query / key row
   static constexpr int kSlabsV = HDV / 64;
@@ -120,7 +120,7 @@ __global__ void gqa_build_items(const int* seq, const int* pos, int rows, int tq
 template <int HDQ, int HDV, bool KV8 = false>
 __global__ void __launch_bounds__((GqaCfg<HDQ, HDV, KV8>::kThreads), 1)
 gqa_attn_kernel(const GqaArgs a, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_kr) {
+                const __grid_constant__ CUtensorMap tm_v) {
   plow::pdl_launch_dependents();
   plow::pdl_wait();
   using Cfg = GqaCfg<HDQ, HDV, KV8>;
@@ -161,7 +161,7 @@ gqa_attn_kernel(const GqaArgs a, const __grid_constant__ CUtensorMap tm_q, const
     *abort_flag = 0;
     *never_flag = 0;
     fence_mbar_init();
-    tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v); tma_prefetch_desc(&tm_kr);
+    tma_prefetch_desc(&tm_q); tma_prefetch_desc(&tm_k); tma_prefetch_desc(&tm_v);
   }
   if (warp == 1) { tmem_alloc(tmem_holder, Cfg::kTmemCols); tmem_relinquish(); }
   tc_fence_before();
@@ -171,12 +171,6 @@ gqa_attn_kernel(const GqaArgs a, const __grid_constant__ CUtensorMap tm_q, const
   const uint32_t tm_s = tmem_base;         // S buffers [0,64) and [64,128); P (bf16 pairs) over the first 32 of each
   const uint32_t tm_o = tmem_base + 128;   // O: HD columns
   const int n_items = *a.n_items;
-  // head-major visiting order (every chunk holds one item per head, no splits): the CTAs running at one time then
-  // work on a handful of heads and share those heads' K / V through L2, instead of touching every head's K / V at once
-  const int n_chunks = a.head_major ? n_items / a.nkv : 0;
-  auto item_at = [&](int it) -> GqaItem {
-    return a.items[a.head_major ? (it % n_chunks) * a.nkv + it / n_chunks : it];
-  };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -184,7 +178,7 @@ gqa_attn_kernel(const GqaArgs a, const __grid_constant__ CUtensorMap tm_q, const
       uint32_t item_it = 0, kv_it = 0;
       bool ok = true;
       for (int it = blockIdx.x; ok && it < n_items; it += gridDim.x, ++item_it) {
-        const GqaItem w = item_at(it);
+        const GqaItem w = a.items[it];
         if (!mbar_wait(q_empty, (item_it & 1) ^ 1, abort_flag)) { *abort_flag = 1; atomicCAS(a.status, 0, PLOW_ERR_STAGE_WAIT | kTagGqa); break; }
         mbar_expect_tx(q_full, Cfg::kQBytes);
         for (int c = 0; c < Cfg::kSlabsQ; ++c) tma_load_3d(q_smem + c * 16384, &tm_q, c * 64, w.kvh * a.group, w.r0, q_full);
@@ -211,12 +205,8 @@ gqa_attn_kernel(const GqaArgs a, const __grid_constant__ CUtensorMap tm_q, const
           }
           uint8_t* st = kv_smem + s * Cfg::kStageBytes;
           mbar_expect_tx(&kv_full[s], Cfg::kStageBytes);
-          for (int c = 0; c < Cfg::kSlabsQ; ++c) {
-            if (c < Cfg::kSlabsQ - a.kr_slabs) tma_load_3d(st + c * 8192, &tm_k, c * 64, w.kvh, page * kGqaPage, &kv_full[s]);
-            else tma_load_3d(st + c * 8192, &tm_kr, (c - (Cfg::kSlabsQ - a.kr_slabs)) * 64, 0, page * kGqaPage, &kv_full[s]);
-          }
-          for (int c = 0; c < Cfg::kSlabsV; ++c)
-            tma_load_3d(st + Cfg::kKBytes + c * 8192, &tm_v, a.v_x0 + c * 64, w.kvh, page * kGqaPage, &kv_full[s]);
+          for (int c = 0; c < Cfg::kSlabsQ; ++c) tma_load_3d(st + c * 8192, &tm_k, c * 64, w.kvh, page * kGqaPage, &kv_full[s]);
+          for (int c = 0; c < Cfg::kSlabsV; ++c) tma_load_3d(st + Cfg::kKBytes + c * 8192, &tm_v, c * 64, w.kvh, page * kGqaPage, &kv_full[s]);
         }
       }
     }
@@ -245,7 +235,7 @@ gqa_attn_kernel(const GqaArgs a, const __grid_constant__ CUtensorMap tm_q, const
         return true;
       };
       for (int it = blockIdx.x; ok && it < n_items; it += gridDim.x, ++item_it) {
-        const GqaItem w = item_at(it);
+        const GqaItem w = a.items[it];
         if (!mbar_wait(q_full, item_it & 1, abort_flag)) { *abort_flag = 1; atomicCAS(a.status, 0, PLOW_ERR_TMA_WAIT | kTagGqa); break; }
         tc_fence_after();
         if (!issue_qk(kv_it, tile_it)) { *abort_flag = 1; break; }
@@ -283,7 +273,7 @@ gqa_attn_kernel(const GqaArgs a, const __grid_constant__ CUtensorMap tm_q, const
     uint32_t kv_it = 0;
     bool ok = true;
     for (int it = blockIdx.x; ok && it < n_items; it += gridDim.x) {
-      const GqaItem w = item_at(it);
+      const GqaItem w = a.items[it];
       const int* pt = a.page_table + static_cast<size_t>(w.slot) * a.max_pages + w.tile0;
       // page numbers of the item's tiles in a shared ring (128 entries, refilled 64 at a time, 64 tiles ahead): the
       // scale fetch of tile i + 2 then starts from a shared-memory read instead of a dependent global load
@@ -368,7 +358,7 @@ gqa_attn_kernel(const GqaArgs a, const __grid_constant__ CUtensorMap tm_q, const
     uint32_t item_it = 0, tile_it = 0;
     bool ok = true;
     for (int it = blockIdx.x; ok && it < n_items; it += gridDim.x, ++item_it) {
-      const GqaItem w = item_at(it);
+      const GqaItem w = a.items[it];
       const int n_valid = w.nt * a.group;
       const bool warp_active = lq * 32 < n_valid;       // whole warp: rows past the chunk are never read
       const int tok = min(li / a.group, w.nt - 1);
@@ -580,6 +570,13 @@ __global__ void rope_kv_kernel(__nv_bfloat16* q_out, const __nv_bfloat16* qkv, i
   const int p = pos[r];
   if (p < 0) return;
   float* buf = rk_smem + wib * hd;
+  // one row, 16 bytes at a time where both sides are aligned for it
+  auto copy_row = [&](__nv_bfloat16* to, const __nv_bfloat16* from) {
+    if (((reinterpret_cast<uintptr_t>(to) | reinterpret_cast<uintptr_t>(from)) & 15) == 0)
+      for (int i = lane; i < hd / 8; i += 32) reinterpret_cast<uint4*>(to)[i] = reinterpret_cast<const uint4*>(from)[i];
+    else
+      for (int i = lane; i < hd; i += 32) to[i] = from[i];
+  };
   // gated attention: every query head is stored as [Q (hd) | gate (hd)]; K and V follow the 2*hd-wide query heads
   const int qw = gate_out ? 2 * hd : hd;
   const __nv_bfloat16* src = qkv + static_cast<size_t>(r) * ld_qkv +
@@ -592,9 +589,7 @@ __global__ void rope_kv_kernel(__nv_bfloat16* q_out, const __nv_bfloat16* qkv, i
   if (h < nq) {
     dst = q_out + (static_cast<size_t>(r) * nq + h) * hd;
     gamma = qn;
-    if (gate_out)
-      for (int i = lane; i < hd / 8; i += 32)
-        reinterpret_cast<uint4*>(gate_out + (static_cast<size_t>(r) * nq + h) * hd)[i] = reinterpret_cast<const uint4*>(src + hd)[i];
+    if (gate_out) copy_row(gate_out + (static_cast<size_t>(r) * nq + h) * hd, src + hd);
   } else {
     const int kh = is_v ? h - nq - nkv : h - nq;
     const int page = page_table[static_cast<size_t>(seq[r]) * max_pages + p / kGqaPage];
@@ -625,7 +620,7 @@ __global__ void rope_kv_kernel(__nv_bfloat16* q_out, const __nv_bfloat16* qkv, i
       store8();
       return;
     }
-    for (int i = lane; i < hd / 8; i += 32) reinterpret_cast<uint4*>(dst)[i] = reinterpret_cast<const uint4*>(src)[i];
+    copy_row(dst, src);
     return;
   }
   float ss = 0.f;
@@ -666,6 +661,98 @@ __global__ void rope_kv_kernel(__nv_bfloat16* q_out, const __nv_bfloat16* qkv, i
   for (int i = rot + lane; i < hd; i += 32) dst[i] = __float2bfloat16(buf[i]);
 }
 
+// The same for heads of 128 whose whole width is rotated: a lane holds two rotation pairs in registers, the row's angles,
+// position and page are read once for `HPW` heads, every access is 4 or 8 bytes a lane.  (With 2-byte accesses through
+// shared memory and a lookup of everything per head, 4096 rows of 48 heads took 82 us against 16 us of traffic.)
+template <int HPW>
+__global__ void __launch_bounds__(256)
+rope_kv128_kernel(__nv_bfloat16* q_out, const __nv_bfloat16* qkv, int ld_qkv, __nv_bfloat16* kc, __nv_bfloat16* vc,
+                  const __nv_bfloat16* qn, const __nv_bfloat16* kn, const float* rope_tab, const int* pos, const int* seq,
+                  const int* page_table, int max_pages, int rows, int nq, int nkv, int pair_mode, int plus_one, float eps,
+                  float* kv_scale) {
+  plow::pdl_launch_dependents();
+  plow::pdl_wait();
+  constexpr int hd = 128;
+  const int lane = threadIdx.x & 31;
+  const int heads = nq + 2 * nkv, groups = (heads + HPW - 1) / HPW;
+  const long long item = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (item >= static_cast<long long>(rows) * groups) return;
+  const int r = static_cast<int>(item / groups), h0 = static_cast<int>(item % groups) * HPW;
+  const int p = pos[r];
+  if (p < 0) return;
+  const float* tab = rope_tab + static_cast<size_t>(p) * hd;
+  const float2 cs = make_float2(tab[2 * lane], tab[2 * lane + 1]), sn = make_float2(tab[64 + 2 * lane], tab[64 + 2 * lane + 1]);
+  const int page = page_table[static_cast<size_t>(seq[r]) * max_pages + p / kGqaPage];
+  const size_t tok = static_cast<size_t>(page) * kGqaPage + p % kGqaPage;
+  // dims of the lane's pairs (x0, y0), (x1, y1): half split (2l, 64 + 2l), (2l + 1, 65 + 2l); interleaved (4l, 4l + 1), ...
+  auto load = [&](const __nv_bfloat16* src, float* v) {
+    uint32_t a, b;
+    if (pair_mode) { const uint2 u = *reinterpret_cast<const uint2*>(src + 4 * lane); a = u.x; b = u.y; }
+    else { a = *reinterpret_cast<const uint32_t*>(src + 2 * lane); b = *reinterpret_cast<const uint32_t*>(src + 64 + 2 * lane); }
+    const __nv_bfloat162 ha = *reinterpret_cast<const __nv_bfloat162*>(&a), hb = *reinterpret_cast<const __nv_bfloat162*>(&b);
+    v[0] = __bfloat162float(ha.x); v[1] = __bfloat162float(ha.y); v[2] = __bfloat162float(hb.x); v[3] = __bfloat162float(hb.y);
+  };
+  auto store = [&](__nv_bfloat16* dst, const float* v) {
+    const __nv_bfloat162 ha = __floats2bfloat162_rn(v[0], v[1]), hb = __floats2bfloat162_rn(v[2], v[3]);
+    const uint32_t a = *reinterpret_cast<const uint32_t*>(&ha), b = *reinterpret_cast<const uint32_t*>(&hb);
+    if (pair_mode) *reinterpret_cast<uint2*>(dst + 4 * lane) = make_uint2(a, b);
+    else { *reinterpret_cast<uint32_t*>(dst + 2 * lane) = a; *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = b; }
+  };
+  float v[HPW][4];
+#pragma unroll
+  for (int i = 0; i < HPW; ++i)
+    if (h0 + i < heads) load(qkv + static_cast<size_t>(r) * ld_qkv + static_cast<size_t>(h0 + i) * hd, v[i]);
+#pragma unroll
+  for (int i = 0; i < HPW; ++i) {
+    const int h = h0 + i;
+    if (h >= heads) break;
+    const bool is_q = h < nq, is_v = h >= nq + nkv;
+    float* x = v[i];
+    const __nv_bfloat16* gamma = is_q ? qn : (is_v ? nullptr : kn);
+    if (gamma) {
+      float ss = x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float rs = rsqrtf(ss / hd + eps);
+      float g[4];
+      load(gamma, g);
+      // the normalised value is rounded to bf16 before the rotation, as the unfused pair would do
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[j] = __bfloat162float(__float2bfloat16(x[j] * rs * (plus_one ? 1.0f + g[j] : g[j])));
+    }
+    if (!is_v) {
+      // half split: x[0], x[2] and x[1], x[3] are pairs; interleaved: x[0], x[1] and x[2], x[3]
+      const float a0 = x[0], b0 = pair_mode ? x[1] : x[2], a1 = pair_mode ? x[2] : x[1], b1 = x[3];
+      const float ra0 = a0 * cs.x - b0 * sn.x, rb0 = b0 * cs.x + a0 * sn.x;
+      const float ra1 = a1 * cs.y - b1 * sn.y, rb1 = b1 * cs.y + a1 * sn.y;
+      x[0] = ra0; x[3] = rb1;
+      x[1] = pair_mode ? rb0 : ra1;
+      x[2] = pair_mode ? ra1 : rb0;
+    }
+    if (is_q) { store(q_out + (static_cast<size_t>(r) * nq + h) * hd, x); continue; }
+    const int kh = is_v ? h - nq - nkv : h - nq;
+    const size_t cell = (tok * nkv + kh) * hd;
+    if (!kv_scale) { store((is_v ? vc : kc) + cell, x); continue; }
+    // e4m3 cell: the finished row (bf16-rounded, as the bf16 cache would hold it) scaled by amax / 448, one scale per cell
+    float amax = 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { x[j] = __bfloat162float(__float2bfloat16(x[j])); amax = fmaxf(amax, fabsf(x[j])); }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    const float sc = fmaxf(amax, 1e-12f) / 448.0f, inv = 1.0f / sc;
+    uint32_t q[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) q[j] = static_cast<uint8_t>(__nv_cvt_float_to_fp8(x[j] * inv, __NV_SATFINITE, __NV_E4M3));
+    uint8_t* d8 = reinterpret_cast<uint8_t*>(is_v ? vc : kc) + cell;
+    if (pair_mode) *reinterpret_cast<uint32_t*>(d8 + 4 * lane) = q[0] | (q[1] << 8) | (q[2] << 16) | (q[3] << 24);
+    else {
+      *reinterpret_cast<uint16_t*>(d8 + 2 * lane) = static_cast<uint16_t>(q[0] | (q[1] << 8));
+      *reinterpret_cast<uint16_t*>(d8 + 64 + 2 * lane) = static_cast<uint16_t>(q[2] | (q[3] << 8));
+    }
+    if (lane == 0) kv_scale[tok * 2 * nkv + (is_v ? nkv : 0) + kh] = sc;
+  }
+}
+
 template <int HD>
 int launch_gqa(const GqaArgs& a, const void* q, const void* kc, const void* vc, int64_t n_pages, int grid, cudaStream_t stream) {
   using Cfg = GqaCfg<HD, HD>;
@@ -678,7 +765,7 @@ int launch_gqa(const GqaArgs& a, const void* q, const void* kc, const void* vc, 
   if (r) return 1300 + r;
   static DeviceOnce attr;
   if (ensure_smem(attr, gqa_attn_kernel<HD, HD>, Cfg::kSmem) != cudaSuccess) return 3000;
-  plow::launch_serial(gqa_attn_kernel<HD, HD>, dim3(grid), dim3(kGqaThreads), Cfg::kSmem, stream, a, tq, tk, tv, tk);
+  plow::launch_serial(gqa_attn_kernel<HD, HD>, dim3(grid), dim3(kGqaThreads), Cfg::kSmem, stream, a, tq, tk, tv);
   return 0;
 }
 
@@ -695,24 +782,7 @@ int launch_gqa8(const GqaArgs& a, const void* q, const void* kc, const void* vc,
   if (r) return 1300 + r;
   static DeviceOnce attr;
   if (ensure_smem(attr, gqa_attn_kernel<HD, HD, true>, Cfg::kSmem) != cudaSuccess) return 3000;
-  plow::launch_serial(gqa_attn_kernel<HD, HD, true>, dim3(grid), dim3(Cfg::kThreads), Cfg::kSmem, stream, a, tq, tk, tv, tk);
-  return 0;
-}
-
-// Materialised multi-head latent attention (prefill): q [rows][heads][192]; kvb [tokens][heads][256] = per head
-// [128 no-position key dims | 128 value dims]; krope [tokens][64] shared by all heads.
-int launch_mla_prefill(const GqaArgs& a, const void* q, const void* kvb, const void* krope, int64_t n_tokens, int grid, cudaStream_t stream) {
-  using Cfg = GqaCfg<192, 128>;
-  CUtensorMap tq, tk, tkr;
-  int r = make_tmap_3d(&tq, q, 2, 192, a.nq, a.rows, 192 * 2, static_cast<uint64_t>(a.nq) * 192 * 2, 1, 128, 128);
-  if (r) return 1100 + r;
-  r = make_tmap_3d(&tk, kvb, 2, 256, a.nkv, static_cast<uint64_t>(n_tokens), 256 * 2, static_cast<uint64_t>(a.nkv) * 256 * 2, 1, kGqaPage, 128);
-  if (r) return 1200 + r;
-  r = make_tmap_3d(&tkr, krope, 2, 64, 1, static_cast<uint64_t>(n_tokens), 64 * 2, 64 * 2, 1, kGqaPage, 128);
-  if (r) return 1300 + r;
-  static DeviceOnce attr;
-  if (ensure_smem(attr, gqa_attn_kernel<192, 128>, Cfg::kSmem) != cudaSuccess) return 3000;
-  plow::launch_serial(gqa_attn_kernel<192, 128>, dim3(grid), dim3(kGqaThreads), Cfg::kSmem, stream, a, tq, tk, tk, tkr);
+  plow::launch_serial(gqa_attn_kernel<HD, HD, true>, dim3(grid), dim3(Cfg::kThreads), Cfg::kSmem, stream, a, tq, tk, tv);
   return 0;
 }
 
@@ -737,6 +807,14 @@ int plow_gqa_attention(const void* q, const void* kc, const void* vc, int64_t n_
   if (hd != 128 && hd != 256) return -3;
   if (kv_scale && hd != 128) return -4;
   const int tq = 128 / group;
+  if (hd == 128 && !kv_scale && max_splits == 1 && rows > kPrefillRows) {
+    PrefillArgs p = {q, kc, vc, nullptr, page_table, seq, pos, items, item_cap, n_items, row_ns, out, status,
+                     n_pages * kGqaPage, rows, nq, nkv, max_pages, window, softmax_scale};
+    const int rc = launch_attn_prefill(p, stream);
+    if (rc) return rc;
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : 4000 + static_cast<int>(e);
+  }
   cudaMemsetAsync(n_items, 0, sizeof(int), stream);
   plow::launch_serial(gqa_build_items, dim3((rows + 255) / 256), dim3(256), 0, stream, seq, pos, rows, tq, nkv, window, tiles_per_split, max_splits,
                                                          static_cast<GqaItem*>(items), n_items, row_ns, item_cap, status);
@@ -745,7 +823,7 @@ int plow_gqa_attention(const void* q, const void* kc, const void* vc, int64_t n_
   a.opart = opart; a.lse = lse; a.out = static_cast<__nv_bfloat16*>(out); a.status = status;
   a.rows = rows; a.nq = nq; a.nkv = nkv; a.group = group; a.max_pages = max_pages; a.max_splits = max_splits; a.window = window;
   a.scale_log2e = softmax_scale * 1.4426950408889634f;
-  a.kr_slabs = 0; a.v_x0 = 0; a.head_major = 0; a.kv_scale = kv_scale;
+  a.kv_scale = kv_scale;
   int grid = sm_count();
   if (item_cap < grid) grid = item_cap;
   int r = kv_scale ? launch_gqa8<128>(a, q, kc, vc, n_pages, grid, stream)
@@ -760,29 +838,19 @@ int plow_gqa_attention(const void* q, const void* kc, const void* vc, int64_t n_
 // Multi-head latent attention over materialised keys / values (prefill).  q bf16 [rows][heads][192] (rotary part
 // already rotated); kvb bf16 [n_tokens][heads][256]; krope bf16 [n_tokens][64]; vpt int32 [n_slots][max_pages]: tile i
 // of slot s covers tokens [64 vpt[s][i], 64 vpt[s][i] + 64) of kvb / krope; seq / pos int32 [rows] (pos < 0: the row is
-// not attended here); out bf16 [rows][heads*128].  Scratch as for plow_gqa_attention (opart / lse with hd = 128).
+// not attended here); out bf16 [rows][heads*128].  Scratch: items (8 ints each, capacity item_cap), n_items (1 int), row_ns
+// int32 [rows].  Keys are never split (a chunk has an item for every head): the split arguments and their scratch are unused.
 int plow_mla_prefill_attention(const void* q, const void* kvb, const void* krope, int64_t n_tokens, const int* vpt, int max_pages,
                                const int* seq, const int* pos, int rows, int heads, int tiles_per_split, int max_splits,
                                void* items, int item_cap, int* n_items, int* row_ns, float* opart, float* lse, void* out,
                                float softmax_scale, int* status, void* stream_) {
   using namespace plow;
-  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   if (rows <= 0 || heads <= 0 || max_splits <= 0 || tiles_per_split <= 0 || n_tokens <= 0) return -1;
-  cudaMemsetAsync(n_items, 0, sizeof(int), stream);
-  plow::launch_serial(gqa_build_items, dim3((rows + 255) / 256), dim3(256), 0, stream, seq, pos, rows, 128, heads, 0, tiles_per_split,
-                      max_splits, static_cast<GqaItem*>(items), n_items, row_ns, item_cap, status);
-  GqaArgs a;
-  a.page_table = vpt; a.pos = pos; a.items = static_cast<const GqaItem*>(items); a.n_items = n_items;
-  a.opart = opart; a.lse = lse; a.out = static_cast<__nv_bfloat16*>(out); a.status = status;
-  a.rows = rows; a.nq = heads; a.nkv = heads; a.group = 1; a.max_pages = max_pages; a.max_splits = max_splits; a.window = 0;
-  a.scale_log2e = softmax_scale * 1.4426950408889634f;
-  a.kr_slabs = 1; a.v_x0 = 128; a.head_major = max_splits == 1 ? 1 : 0; a.kv_scale = nullptr;
-  int grid = sm_count();
-  if (item_cap < grid) grid = item_cap;
-  int r = launch_mla_prefill(a, q, kvb, krope, n_tokens, grid, stream);
-  if (r) return r;
-  if (max_splits > 1)
-    plow::launch_serial(gqa_merge_kernel, dim3(rows, heads), dim3(128), 0, stream, opart, lse, row_ns, heads, max_splits, 128, static_cast<__nv_bfloat16*>(out));
+  (void)opart; (void)lse;
+  PrefillArgs p = {q, kvb, kvb, krope, vpt, seq, pos, items, item_cap, n_items, row_ns, out, status,
+                   n_tokens, rows, heads, heads, max_pages, 0, softmax_scale};
+  const int rc = launch_attn_prefill(p, reinterpret_cast<cudaStream_t>(stream_));
+  if (rc) return rc;
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 4000 + static_cast<int>(e);
 }
@@ -797,6 +865,23 @@ int plow_rope_kv(void* q_out, const void* qkv, int ld_qkv, void* kc, void* vc, c
                  float* kv_scale, void* stream_) {
   using namespace plow;
   if (rows <= 0 || hd % 8 || rot > hd || rot % 2) return -1;
+  // whole-width rotation of 128-wide heads with rows aligned for 8-byte access; gated attention keeps the general kernel
+  const uintptr_t at = reinterpret_cast<uintptr_t>(q_out) | reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(kc) |
+                       reinterpret_cast<uintptr_t>(vc) | reinterpret_cast<uintptr_t>(qn) | reinterpret_cast<uintptr_t>(kn);
+  if (hd == 128 && rot == 128 && !gate_out && (at & 7) == 0 && ld_qkv % 4 == 0) {
+    const int heads = nq + 2 * nkv;
+    auto run = [&](auto kern, int hpw) {
+      const long long warps = static_cast<long long>(rows) * ((heads + hpw - 1) / hpw);
+      plow::launch_serial(kern, dim3(static_cast<unsigned>((warps + 7) / 8)), dim3(256), 0, reinterpret_cast<cudaStream_t>(stream_),
+          static_cast<__nv_bfloat16*>(q_out), static_cast<const __nv_bfloat16*>(qkv), ld_qkv, static_cast<__nv_bfloat16*>(kc),
+          static_cast<__nv_bfloat16*>(vc), static_cast<const __nv_bfloat16*>(qn), static_cast<const __nv_bfloat16*>(kn), rope_tab, pos, seq,
+          page_table, max_pages, rows, nq, nkv, pair_mode, plus_one, eps, kv_scale);
+    };
+    // eight heads a warp once that leaves every SM a block
+    if (static_cast<long long>(rows) * heads >= 148 * 8 * 8) run(rope_kv128_kernel<8>, 8); else run(rope_kv128_kernel<1>, 1);
+    cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : 4000 + static_cast<int>(e);
+  }
   const long long items = static_cast<long long>(rows) * (nq + 2 * nkv);
   const int wpb = 8;
   plow::launch_serial(rope_kv_kernel, dim3(static_cast<unsigned>((items + wpb - 1) / wpb)), dim3(wpb * 32), wpb * hd * sizeof(float), reinterpret_cast<cudaStream_t>(stream_), 

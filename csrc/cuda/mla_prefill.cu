@@ -10,7 +10,7 @@
 //            dequantised to bf16 when the up-projection weight is bf16.  The rotary key part is dequantised to bf16.
 //   GEMM   : kvb[token][head][nope | v] = latent . W_kv_b^T (the library's GEMM)
 //   rope   : the rotary part of the new query rows, in place
-//   attend : the tcgen05 flash kernel of attn_gqa.cu with 192-wide keys and 128-wide values
+//   attend : the tcgen05 flash kernel of attn_prefill.cu with 192-wide keys and 128-wide values
 //
 // Reference counterpart: crates/devgen/src/mla.rs (prefill expands the latent through kv_b_proj before attention).
 #include <cuda_bf16.h>
@@ -101,6 +101,36 @@ __global__ void mla_q_rope_kernel(__nv_bfloat16* q, int pitch, const float* rope
   }
 }
 
+// The same for 64 rotary dims in interleaved pairs: lane i owns pair i (4 bytes), the row's angles are read once for eight
+// heads whose loads are all in flight (2048 rows of 128 heads: 46 us with 2-byte accesses and a lookup per head; the
+// traffic takes 10).
+__global__ void __launch_bounds__(256)
+mla_q_rope64_kernel(__nv_bfloat16* q, int pitch, const float* rope_tab, const int* pos, int T, int heads, int nope) {
+  plow::pdl_launch_dependents();
+  plow::pdl_wait();
+  constexpr int kHeads = 8;
+  const int lane = threadIdx.x & 31;
+  const int groups = (heads + kHeads - 1) / kHeads;
+  const long long item = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (item >= static_cast<long long>(T) * groups) return;
+  const int r = static_cast<int>(item / groups), h0 = static_cast<int>(item % groups) * kHeads;
+  const int p = pos[r];
+  if (p < 0) return;
+  const float* tab = rope_tab + static_cast<size_t>(p) * 64;
+  const float c = tab[lane], s = tab[32 + lane];
+  __nv_bfloat16* v = q + static_cast<size_t>(r) * pitch + static_cast<size_t>(h0) * (nope + 64) + nope + 2 * lane;
+  __nv_bfloat162 x[kHeads];
+#pragma unroll
+  for (int i = 0; i < kHeads; ++i)
+    if (h0 + i < heads) x[i] = *reinterpret_cast<const __nv_bfloat162*>(v + static_cast<size_t>(i) * (nope + 64));
+#pragma unroll
+  for (int i = 0; i < kHeads; ++i)
+    if (h0 + i < heads) {
+      const float a = __bfloat162float(x[i].x), b = __bfloat162float(x[i].y);
+      *reinterpret_cast<__nv_bfloat162*>(v + static_cast<size_t>(i) * (nope + 64)) = __floats2bfloat162_rn(a * c - b * s, b * c + a * s);
+    }
+}
+
 }  // namespace
 
 extern "C" {
@@ -125,6 +155,13 @@ int plow_mla_q_rope(void* q, int pitch, const float* rope_tab, const int* pos, i
                     int pair_mode, void* stream) {
   if (T <= 0) return 0;
   const int wpb = 8;
+  if (rope == 64 && pair_mode && (reinterpret_cast<uintptr_t>(q) & 3) == 0 && pitch % 2 == 0 && nope % 2 == 0) {
+    const long long warps = static_cast<long long>(T) * ((heads + 7) / 8);
+    plow::launch_serial(mla_q_rope64_kernel, dim3(static_cast<unsigned>((warps + wpb - 1) / wpb)), dim3(wpb * 32), 0,
+                        static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(q), pitch, rope_tab, pos, T, heads, nope);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : 4000 + static_cast<int>(e);
+  }
   const long long items = static_cast<long long>(T) * heads;
   plow::launch_serial(mla_q_rope_kernel, dim3(static_cast<unsigned>((items + wpb - 1) / wpb)), dim3(wpb * 32), 0,
                       static_cast<cudaStream_t>(stream), static_cast<__nv_bfloat16*>(q), pitch, rope_tab, pos, T, heads, nope,
