@@ -34,6 +34,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
+#include "attn_decode.cuh"
 #include "attn_prefill.h"
 #include "ptx.cuh"
 #include "tmap.cuh"
@@ -63,6 +64,9 @@ struct GqaArgs {
   int rows, nq, nkv, group, max_pages, max_splits, window;
   float scale_log2e;
   const float* kv_scale;   // e4m3 cache: [n_pages][64][2 * nkv] f32, k scales then v scales of a token
+  void* dec;               // scratch of attn_decode.cuh; null: this call is no candidate
+  const __nv_bfloat16* q;
+  const int* seq;
 };
 
 // HDQ = width of a query / key row, HDV = width of a value row.
@@ -81,7 +85,7 @@ template <int HDQ, int HDV, bool KV8 = false> struct GqaCfg {
   // per operand stage: 64 S-column and 64 P-column factors; then a ring of 128 page numbers for the converter warps
   static constexpr int kColBytes = KV8 ? kStages * 128 * 4 + 128 * 4 : 0;
   static constexpr int kSmem = 1024 + kQBytes + kStages * kStageBytes + kRawBytes + kColBytes + 1024;
-  static constexpr int kThreads = KV8 ? kGqaThreads8 : kGqaThreads;
+  static constexpr int kThreads = KV8 ? kGqaThreads8 : (HDQ == 128 ? kDecThreads : kGqaThreads);
   static constexpr int kTmemCols = HDV <= 128 ? 256 : 512; // S: 2 x 64, O: HDV
   static_assert(kStages >= 2, "K/V stages do not fit");
   static_assert(kSmem <= 227 * 1024, "shared memory budget");
@@ -117,12 +121,73 @@ __global__ void gqa_build_items(const int* seq, const int* pos, int rows, int tq
   }
 }
 
+// Work of a call of up to kDecMaxRows rows, by one block.  Every row a sequence of its own (a decode step): the pages of the
+// step as one line for attn_decode.cuh; otherwise the items of the tile kernel as above.
+__global__ void __launch_bounds__(kDecMaxRows)
+gqa_plan_small(const int* seq, const int* pos, int rows, int tq, int nkv, int window, int tiles_per_split, int max_splits, GqaItem* items,
+               int* n_items, int* row_ns, int cap, void* dec, int* status) {
+  plow::pdl_launch_dependents();
+  plow::pdl_wait();
+  __shared__ int warp_sum[kDecMaxRows / 32], n_sh;
+  const DecScratch sc(dec, rows, nkv);
+  const int r = threadIdx.x, lane = r & 31, warp = r >> 5;
+  const bool live = r < rows && pos[r] >= 0;
+  const bool joins = live && r > 0 && pos[r - 1] >= 0 && seq[r] == seq[r - 1] && pos[r] == pos[r - 1] + 1;
+  if (r == 0) n_sh = 0;
+  const bool decode = !__syncthreads_or(joins);
+  if (decode) {
+    const int hi = live ? pos[r] : 0, lo = window > 0 ? max(0, hi - window + 1) : 0;
+    const int n = live ? (hi / kGqaPage - lo / kGqaPage + 1) * nkv : 0;
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += t; }
+    if (lane == 31) warp_sum[warp] = incl;
+    __syncthreads();
+    int base = 0, total = 0;
+    for (int w = 0; w < kDecMaxRows / 32; ++w) { if (w < warp) base += warp_sum[w]; total += warp_sum[w]; }
+    if (r < rows) sc.prefix[r] = base + incl - n;
+    if (r == 0) { sc.plan[0] = 1; sc.plan[1] = total; sc.prefix[rows] = total; *n_items = 0; }
+    for (int i = r; i < rows * nkv; i += kDecMaxRows) sc.arrived[i] = 0;
+    if (r < rows) row_ns[r] = live ? 1 : 0;
+    return;
+  }
+  if (r < rows && !live) row_ns[r] = 0;
+  if (live && (!joins || r % tq == 0)) {
+    int nt = 1;
+    while ((r + nt) % tq != 0 && r + nt < rows && seq[r + nt] == seq[r] && pos[r + nt] == pos[r + nt - 1] + 1) ++nt;
+    const int hi = pos[r + nt - 1];
+    const int lo = window > 0 ? max(0, pos[r] - window + 1) : 0;
+    const int tile_lo = lo / kGqaPage;
+    const int tiles = hi / kGqaPage + 1 - tile_lo;
+    int ns = min(max_splits, (tiles + tiles_per_split - 1) / tiles_per_split);
+    const int per = (tiles + ns - 1) / ns;
+    ns = (tiles + per - 1) / per;
+    for (int j = 0; j < nt; ++j) row_ns[r + j] = ns;
+    const int base = atomicAdd(&n_sh, nkv * ns);
+    if (base + nkv * ns > cap) { atomicCAS(status, 0, PLOW_ERR_BOUNDS | kTagGqa); }
+    else
+      for (int h = 0; h < nkv; ++h)
+        for (int s = 0; s < ns; ++s)
+          items[base + h * ns + s] = GqaItem{r, nt, h, s, tile_lo + s * per, min(per, tiles - s * per), seq[r], ns};
+  }
+  __syncthreads();
+  if (r == 0) { *n_items = min(n_sh, cap); sc.plan[0] = 0; }
+}
+
 template <int HDQ, int HDV, bool KV8 = false>
 __global__ void __launch_bounds__((GqaCfg<HDQ, HDV, KV8>::kThreads), 1)
 gqa_attn_kernel(const GqaArgs a, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v) {
   plow::pdl_launch_dependents();
   plow::pdl_wait();
+  if constexpr (HDQ == 128) {
+    // a decode step: the streaming form (the plan kernel decided)
+    if (a.dec && *static_cast<const int*>(a.dec) == 1) {
+      const DecArgs d = {a.dec, a.q, a.page_table, a.pos, a.seq, a.kv_scale, a.out, a.status, a.rows, a.nq, a.nkv, a.group, a.max_pages, a.window, a.scale_log2e};
+      gqa_decode_body<KV8>(d, &tm_k, &tm_v);
+      return;
+    }
+  }
   using Cfg = GqaCfg<HDQ, HDV, KV8>;
   constexpr int HD = HDV;      // width of the accumulator rows
   extern __shared__ uint8_t smem_raw[];
@@ -350,7 +415,7 @@ gqa_attn_kernel(const GqaArgs a, const __grid_constant__ CUtensorMap tm_q, const
         if (ok && i + 2 < w.ntiles) ok = tile_step(i + 2, sl[2], sl[1]);
       }
     }
-  } else {
+  } else if (warp < 6) {
     // ------------------------------------------------------------------ softmax / epilogue warps
     const int lq = warp & 3;           // TMEM lane quarter this warp may access
     const int li = lq * 32 + lane;     // row of the tile: token li / group, query head li % group
@@ -756,6 +821,8 @@ rope_kv128_kernel(__nv_bfloat16* q_out, const __nv_bfloat16* qkv, int ld_qkv, __
 template <int HD>
 int launch_gqa(const GqaArgs& a, const void* q, const void* kc, const void* vc, int64_t n_pages, int grid, cudaStream_t stream) {
   using Cfg = GqaCfg<HD, HD>;
+  constexpr int kSmem = HD == 128 ? (Cfg::kSmem > DecCfg<false>::smem(kDecMaxGroup) ? Cfg::kSmem : DecCfg<false>::smem(kDecMaxGroup)) : Cfg::kSmem;
+  static_assert(kSmem <= 227 * 1024, "shared memory budget");
   CUtensorMap tq, tk, tv;
   int r = make_tmap_3d(&tq, q, 2, HD, a.nq, a.rows, HD * 2, static_cast<uint64_t>(a.nq) * HD * 2, a.group, 128 / a.group, 128);
   if (r) return 1100 + r;
@@ -764,8 +831,8 @@ int launch_gqa(const GqaArgs& a, const void* q, const void* kc, const void* vc, 
   r = make_tmap_3d(&tv, vc, 2, HD, a.nkv, static_cast<uint64_t>(n_pages) * kGqaPage, HD * 2, static_cast<uint64_t>(a.nkv) * HD * 2, 1, kGqaPage, 128);
   if (r) return 1300 + r;
   static DeviceOnce attr;
-  if (ensure_smem(attr, gqa_attn_kernel<HD, HD>, Cfg::kSmem) != cudaSuccess) return 3000;
-  plow::launch_serial(gqa_attn_kernel<HD, HD>, dim3(grid), dim3(kGqaThreads), Cfg::kSmem, stream, a, tq, tk, tv);
+  if (ensure_smem(attr, gqa_attn_kernel<HD, HD>, kSmem) != cudaSuccess) return 3000;
+  plow::launch_serial(gqa_attn_kernel<HD, HD>, dim3(grid), dim3(Cfg::kThreads), kSmem, stream, a, tq, tk, tv);
   return 0;
 }
 
@@ -773,6 +840,7 @@ int launch_gqa(const GqaArgs& a, const void* q, const void* kc, const void* vc, 
 template <int HD>
 int launch_gqa8(const GqaArgs& a, const void* q, const void* kc, const void* vc, int64_t n_pages, int grid, cudaStream_t stream) {
   using Cfg = GqaCfg<HD, HD, true>;
+  static_assert(DecCfg<true>::smem(kDecMaxGroup) <= Cfg::kSmem, "the decode body fits the tile kernel's shared memory");
   CUtensorMap tq, tk, tv;
   int r = make_tmap_3d(&tq, q, 2, HD, a.nq, a.rows, HD * 2, static_cast<uint64_t>(a.nq) * HD * 2, a.group, 128 / a.group, 128);
   if (r) return 1100 + r;
@@ -795,10 +863,16 @@ extern "C" {
 // row_ns int32 [rows], opart f32 [rows][nq][max_splits][hd], lse f32 [rows][nq][max_splits].
 // kv_scale != null: kc / vc are e4m3 bytes with one f32 scale per (token, kv head) in kv_scale [n_pages][64][2*nkv]
 // (k scales, then v scales); head dim 128 only.
+// Bytes of the optional scratch `dec` of plow_gqa_attention for calls of `rows` rows; 0: such calls use none.
+int64_t plow_gqa_decode_scratch_bytes(int rows, int nq, int nkv, int hd) {
+  if (rows <= 0 || rows > plow::kDecMaxRows || hd != 128 || nkv <= 0 || nq % nkv || nq / nkv > plow::kDecMaxGroup) return 0;
+  return plow::DecScratch::bytes(rows, nkv);
+}
+
 int plow_gqa_attention(const void* q, const void* kc, const void* vc, int64_t n_pages, const int* page_table,
                        int max_pages, const int* seq, const int* pos, int rows, int nq, int nkv, int hd, int window,
                        int tiles_per_split, int max_splits, void* items, int item_cap, int* n_items, int* row_ns,
-                       float* opart, float* lse, void* out, float softmax_scale, const float* kv_scale, int* status, void* stream_) {
+                       float* opart, float* lse, void* out, float softmax_scale, const float* kv_scale, void* dec, int* status, void* stream_) {
   using namespace plow;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   if (rows <= 0 || nq <= 0 || nkv <= 0 || nq % nkv || max_splits <= 0 || tiles_per_split <= 0) return -1;
@@ -815,17 +889,26 @@ int plow_gqa_attention(const void* q, const void* kc, const void* vc, int64_t n_
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : 4000 + static_cast<int>(e);
   }
-  cudaMemsetAsync(n_items, 0, sizeof(int), stream);
-  plow::launch_serial(gqa_build_items, dim3((rows + 255) / 256), dim3(256), 0, stream, seq, pos, rows, tq, nkv, window, tiles_per_split, max_splits,
-                                                         static_cast<GqaItem*>(items), n_items, row_ns, item_cap, status);
+  // small calls: the plan kernel finds out on the device whether this is a decode step
+  if (rows > kDecMaxRows || hd != 128 || group > kDecMaxGroup) dec = nullptr;
+  if (dec) {
+    plow::launch_serial(gqa_plan_small, dim3(1), dim3(kDecMaxRows), 0, stream, seq, pos, rows, tq, nkv, window, tiles_per_split, max_splits,
+                        static_cast<GqaItem*>(items), n_items, row_ns, item_cap, dec, status);
+  } else {
+    cudaMemsetAsync(n_items, 0, sizeof(int), stream);
+    plow::launch_serial(gqa_build_items, dim3((rows + 255) / 256), dim3(256), 0, stream, seq, pos, rows, tq, nkv, window, tiles_per_split, max_splits,
+                        static_cast<GqaItem*>(items), n_items, row_ns, item_cap, status);
+  }
   GqaArgs a;
+  a.dec = dec; a.q = static_cast<const __nv_bfloat16*>(q); a.seq = seq;
   a.page_table = page_table; a.pos = pos; a.items = static_cast<const GqaItem*>(items); a.n_items = n_items;
   a.opart = opart; a.lse = lse; a.out = static_cast<__nv_bfloat16*>(out); a.status = status;
   a.rows = rows; a.nq = nq; a.nkv = nkv; a.group = group; a.max_pages = max_pages; a.max_splits = max_splits; a.window = window;
   a.scale_log2e = softmax_scale * 1.4426950408889634f;
   a.kv_scale = kv_scale;
   int grid = sm_count();
-  if (item_cap < grid) grid = item_cap;
+  if (dec && grid > kDecMaxCtas) grid = kDecMaxCtas;
+  if (!dec && item_cap < grid) grid = item_cap;
   int r = kv_scale ? launch_gqa8<128>(a, q, kc, vc, n_pages, grid, stream)
           : hd == 128 ? launch_gqa<128>(a, q, kc, vc, n_pages, grid, stream) : launch_gqa<256>(a, q, kc, vc, n_pages, grid, stream);
   if (r) return r;

@@ -54,6 +54,9 @@ class AttnWorkspace:
             self.lse = torch.empty(rows, nq, max_splits, dtype=torch.float32, device=device)
         else:
             self.opart = self.lse = None
+        # decode steps stream the cache in equal pieces (csrc/cuda/attn_decode.cuh): plan, arrival counts, partials
+        dec = int(native.cuda_lib().plow_gqa_decode_scratch_bytes(rows, nq, nkv, hd))
+        self.dec_rows, self.dec = (rows, torch.empty(dec, dtype=torch.uint8, device=device)) if dec else (0, None)
 
 
 def attention(q, kc, vc, page_table, seq, pos, ws: AttnWorkspace, scale=None, window=0, out=None, kv_scale=None):
@@ -66,7 +69,7 @@ def attention(q, kc, vc, page_table, seq, pos, ws: AttnWorkspace, scale=None, wi
     native.call("plow_gqa_attention", q, kc, vc, kc.shape[0], page_table, page_table.shape[1], seq, pos, rows, nq, nkv, hd,
                 int(window), ws.tiles_per_split, ws.max_splits, ws.items, ws.item_cap, ws.n_items, ws.row_ns,
                 ws.opart, ws.lse, out, float(scale if scale is not None else 1.0 / math.sqrt(hd)), kv_scale,
-                native.status_word(q.device))
+                ws.dec if rows <= ws.dec_rows else None, native.status_word(q.device))
     return out
 
 

@@ -57,6 +57,8 @@ def cuda_lib() -> C.CDLL:
     lib = C.CDLL(str(_ensure_built("libplow_cuda.so")), mode=C.RTLD_GLOBAL)
     lib.plow_gemm.argtypes = [C.POINTER(GemmDesc), C.c_void_p]
     lib.plow_gemm.restype = C.c_int
+    lib.plow_gqa_decode_scratch_bytes.argtypes = [C.c_int32] * 4
+    lib.plow_gqa_decode_scratch_bytes.restype = C.c_int64
     lib.plow_gdn_scratch_bytes.argtypes = [C.c_int32] * 3
     lib.plow_gdn_scratch_bytes.restype = C.c_int64
     return lib
@@ -148,7 +150,7 @@ _SIGS = {
     "plow_gdn": "ppppipi" "ppppp" "iiiiipp",
     "plow_gated_norm": "pppiipiiifp",
     "plow_sigmoid_gate": "ppplp",
-    "plow_gqa_attention": "ppplpipp" "iiiiiii" "pi" "ppppp" "fppp",
+    "plow_gqa_attention": "ppplpipp" "iiiiiii" "pi" "ppppp" "fpppp",
     "plow_rope_kv": "ppi" "pppppppp" "i" "iiiiiii" "fppp",
     "plow_mla_prefill_attention": "ppplpipp" "iiii" "pi" "ppppp" "fpp",
     "plow_mla_latent_gather": "ppipppppp" "ipiiiip",

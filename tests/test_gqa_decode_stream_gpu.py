@@ -1,0 +1,70 @@
+"""Streaming decode form of the grouped-query attention: sequences from one token up, pages cut between CTAs anywhere, idle
+rows, head ratios, sliding windows, both cache types; calls that are no decode step keep the tile form."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(lens, nq, nkv, kv8, seed, idle=()):
+    from plow_b200.ops import gqa
+    hd, dev = 128, "cuda"
+    g = torch.Generator(device=dev).manual_seed(seed)
+    rows, per = len(lens), (max(lens) + 63) // 64
+    n_pages = rows * per + 1
+    kc = (torch.randn(n_pages, 64, nkv, hd, device=dev, generator=g) * 2).bfloat16()
+    vc = torch.randn(n_pages, 64, nkv, hd, device=dev, generator=g).bfloat16()
+    pt = torch.randperm(n_pages, device=dev, generator=g).int()[: rows * per].view(rows, per).contiguous()
+    pos = torch.tensor(lens, dtype=torch.int32, device=dev) - 1
+    for r in idle:
+        pos[r] = -1
+    seq = torch.randperm(rows, device=dev, generator=g).int()
+    q = torch.randn(rows, nq, hd, device=dev, generator=g).bfloat16()
+    if not kv8:
+        return q, kc, vc, pt, seq, pos, None, kc, vc
+    k8, ks = gqa.quant_cache(kc)
+    v8, vs = gqa.quant_cache(vc)
+    return q, k8, v8, pt, seq, pos, torch.cat([ks, vs], -1).contiguous(), k8.float() * ks[..., None], v8.float() * vs[..., None]
+
+
+@pytest.mark.parametrize("kv8", [False, True])
+@pytest.mark.parametrize("lens,nq,nkv,window,idle", [
+    ([1], 32, 8, 0, ()), ([1, 2, 63, 64, 65, 127, 128, 129], 8, 8, 0, (3,)), ([5000], 32, 8, 0, ()), ([4000, 1, 1, 17], 8, 1, 0, (0, 2)),
+    ([100 + 37 * i for i in range(64)], 32, 8, 0, (0, 31, 63)), ([3000, 700, 70], 16, 4, 200, ()), ([513] * 256, 4, 2, 0, ()),
+    ([1200, 800], 8, 4, 64, ()), ([40, 40, 40], 32, 8, 0, (0, 1, 2))])
+def test_decode_stream(lens, nq, nkv, window, idle, kv8):
+    from plow_b200.ops import gqa, native
+    q, kc, vc, pt, seq, pos, ks, kd, vd = _case(lens, nq, nkv, kv8, len(lens) + sum(lens) % 97, idle)
+    rows = len(lens)
+    ws = gqa.AttnWorkspace(rows, nq, nkv, 128, max(lens), "cuda")
+    assert ws.dec is not None
+    ref = gqa.reference(q, kd, vd, pt, seq, pos, window=window)
+    for _ in range(2):                         # the arrival counts are set up anew by every call
+        out = torch.full((rows, nq * 128), 7.0, device="cuda").bfloat16()
+        gqa.attention(q, kc, vc, pt, seq, pos, ws, window=window, out=out, kv_scale=ks)
+        torch.cuda.synchronize()
+        native.check_status()
+        live = pos >= 0
+        if live.any():
+            rel = (out[live].float() - ref[live]).norm() / ref[live].norm()
+            assert rel < 6e-3, rel             # bf16 probabilities and result
+        assert (out[~live] == 7.0).all()
+
+
+def test_decode_workspace_serves_fewer_rows_and_other_calls():
+    """One workspace: a decode step of fewer rows than it was made for, then a chunk of one sequence, then a step again."""
+    from plow_b200.ops import gqa, native
+    nq, nkv = 32, 8
+    q, kc, vc, pt, seq, pos, _, _, _ = _case([300 + 11 * i for i in range(40)], nq, nkv, False, 3)
+    ws = gqa.AttnWorkspace(48, nq, nkv, 128, 1024, "cuda")
+    for _ in range(2):
+        out = gqa.attention(q[:9], kc, vc, pt, seq[:9], pos[:9], ws)
+        ref = gqa.reference(q[:9], kc, vc, pt, seq[:9], pos[:9])
+        assert (out.float() - ref).norm() / ref.norm() < 6e-3
+        cs, cp = torch.full((40,), 5, dtype=torch.int32, device="cuda"), torch.arange(250, 290, dtype=torch.int32, device="cuda")
+        out = gqa.attention(q, kc, vc, pt, cs, cp, ws)
+        ref = gqa.reference(q, kc, vc, pt, cs, cp)
+        assert (out.float() - ref).norm() / ref.norm() < 6e-3
+    native.check_status()
