@@ -7,21 +7,29 @@
 // e4m3 cache has to be rewritten as bf16 tiles in shared memory (268 us for half the traffic).  Here:
 //   * all (row, kv head, page) triples of the step form one line, cut into equal pieces, one per CTA: every SM streams the
 //     same number of pages.  A (row, kv head) that is cut leaves f32 partials; the CTA that finishes it last folds them.
-//   * one warp feeds a ring of pages (TMA; the e4m3 scales by 4-byte cp.async), eight warps consume: four share a page, 16
-//     tokens each, so two pages are in work at a time.  S = Q K^T and O += P V are m16n8k16 warp MMAs with the heads as
-//     rows; every warp keeps its own running maximum, sum and O, merged through shared memory when a piece ends.
-//   * e4m3 elements become bf16 in registers: the byte s.eeee.mmm placed as s.0000eeee.mmm0000 is value * 2^-120, four
-//     integer instructions per pair; key scales multiply S, value scales P, and the powers of two go with them.  The k index
-//     of an MMA may be any permutation as long as both operands agree, so a lane takes 16 consecutive bytes of a row.
+//   * one warp feeds a ring of pages (TMA; the e4m3 scales by 4-byte cp.async), eight warps consume: two share a page, 32
+//     tokens each, so four pages are in work at a time.  S = Q K^T (heads as rows) and O^T += V^T P^T (heads as columns) are
+//     m16n8k16 warp MMAs: the accumulators of S are the B operand of the other one as they stand.  Every warp keeps its own
+//     running maximum, sum and O, merged through shared memory by three other
+//     warps when a piece ends (merged by the consumers themselves, CTAs with many short sequences took a third longer).
+//   * e4m3 elements become f16 in registers, one conversion per pair (as bf16, by integer instructions, a pair took four and
+//     the ALU pipe half the time); key scales multiply S, value scales P.  Q is scaled by a power of two into f16, which holds
+//     every bf16 down to 2^-28 of the row's largest exactly; the running maximum is taken of score + log2(value scale), so
+//     P times its value scale stays in f16's range, where it has three more bits than in bf16.  The k index of an MMA may be
+//     any permutation as long as both operands agree, so a lane takes 16 consecutive bytes of a row.
+// 64 sequences of 512 .. 4352 tokens, 32 / 8 heads, with the rotary writer: bf16 117 us (tile form 160 .. 169), e4m3 103 us
+// (252 .. 263).  bf16 is at the stream rate; e4m3 is bound by the latency chains of its eight warps.
 // The rates of mma.sync suffice by far (64 of 356 clocks per 16 tokens and SM).
 #pragma once
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
+#include <cuda_fp8.h>
 
 #include "ptx.cuh"
 
 namespace plow {
 
-constexpr int kDecThreads = 320;          // 8 consumer warps, the producer warp, one idle
+constexpr int kDecThreads = 384;          // 8 consumer warps, the producer warp, 3 merge warps
 constexpr int kDecMaxCtas = 160;
 constexpr int kDecMaxGroup = 8;
 constexpr int kDecMaxRows = 256;
@@ -58,16 +66,16 @@ struct DecArgs {
 };
 
 template <bool KV8> struct DecCfg {
-  // Even: stage s then always belongs to the same four warps.  With an odd ring a group would wait for every other phase of a
+  // A multiple of four: stage s then always belongs to the same two warps.  Otherwise a group would wait for some phases of a
   // stage only, and a parity wait cannot tell a phase from the one two before it.
   static constexpr int kStages = KV8 ? 8 : 4;
-  static_assert(kStages % 2 == 0, "a stage belongs to one group of warps");
+  static_assert(kStages % 4 == 0, "a stage belongs to one group of warps");
   static constexpr int kTile = KV8 ? 8192 : 16384;               // one page of keys or values of a head
   static constexpr int kStage = 2 * kTile + (KV8 ? 512 : 0);     // + 64 key and 64 value scales
-  // ring, control, then the merge area: [8 warps][heads][132] f32
+  // ring, control, then two merge areas: [8 warps][heads][132] f32
   static constexpr int kStageStride = (kStage + 1023) / 1024 * 1024;
   static constexpr int kRing = kStages * kStageStride;
-  static constexpr int smem(int group) { return 1024 + kRing + 4096 + 8 * group * 132 * 4; }
+  static constexpr int smem(int group) { return 1024 + kRing + 4096 + 2 * 8 * group * 132 * 4; }
 };
 
 __device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t* r) {
@@ -81,10 +89,21 @@ __device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, uint32_t b
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ void mma_f16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// two e4m3 bytes -> f16x2 (exact)
+__device__ __forceinline__ uint32_t e4m3x2_to_f16(uint32_t x) {
+  const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2(static_cast<__nv_fp8x2_storage_t>(x & 0xffffu), __NV_E4M3);
+  return h.x | (static_cast<uint32_t>(h.y) << 16);
+}
+__device__ __forceinline__ uint32_t f16x2(float a, float b) {
+  const __half2 h = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
 __device__ __forceinline__ float dec_ex2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
-// two e4m3 bytes in the high bytes of two 16-bit lanes -> bf16x2 of value * 2^-120
-__device__ __forceinline__ uint32_t e4m3_lanes_to_bf16(uint32_t x) { return (x & 0x80008000u) | ((x >> 4) & 0x07f007f0u); }
-
 template <bool KV8>
 __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const CUtensorMap* tm_v) {
   using Cfg = DecCfg<KV8>;
@@ -94,17 +113,20 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
   uint8_t* ctrl = ring + Cfg::kRing;
   uint64_t* full = reinterpret_cast<uint64_t*>(ctrl);        // [kS]
   uint64_t* empty = full + kS;                               // [kS]
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + kS);
+  uint64_t* area_full = empty + kS;                          // [2]
+  uint64_t* area_free = area_full + 2;                       // [2]
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(area_free + 2);
   int* last_flag = const_cast<int*>(abort_flag) + 1;
   int* prefix = reinterpret_cast<int*>(ctrl + 512);          // [rows + 1]
-  float* area = reinterpret_cast<float*>(ctrl + 4096);       // [8][group][132]: O, m, l
+  float* area = reinterpret_cast<float*>(ctrl + 4096);       // [2][8][group][132]: O, m, l
   const DecScratch sc(a.scratch, a.rows, a.nkv);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int T = sc.plan[1];
   const int G = min(static_cast<int>(gridDim.x), T);
   if (static_cast<int>(blockIdx.x) >= G) return;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kS; ++s) { mbar_init(&full[s], KV8 ? 33 : 1); mbar_init(&empty[s], 4); }
+    for (int s = 0; s < kS; ++s) { mbar_init(&full[s], KV8 ? 33 : 1); mbar_init(&empty[s], 2); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&area_full[i], 8); mbar_init(&area_free[i], 3); }
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -177,16 +199,17 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
     if (KV8) asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp < 8) {
     // ------------------------------------------------------------------ consumers
-    const int duo = warp >> 2, tok0 = (warp & 3) * 16;       // which of two pages in turn, which 16 of its tokens
+    const int group = warp >> 1, tok0 = (warp & 1) * 32;     // which of four pages in turn, which 32 of its tokens
     const int g = lane >> 2, c4 = lane & 3;
-    uint32_t k0 = 0;                                         // pages of the pieces before
+    uint32_t k0 = 0, n_piece = 0;                            // pages of the pieces before, pieces
     bool ok = true;
-    for (int p = p0; p < p1;) {
+    for (int p = p0; ok && p < p1; ++n_piece) {
       const Piece c = piece_at(p);
-      // Q fragments: MMA rows 0 .. 7 are the heads of this kv head, rows 8 .. 15 stay zero.  k-step s covers dims 16 s + {2 c4, 2 c4 + 1, + 8, + 9};
-      // for e4m3 dims 64 (s / 4) + 16 c4 + 4 (s % 4) + {0, 1, 2, 3} in the same places
+      // Q fragments: MMA rows 0 .. 7 are the heads of this kv head, rows 8 .. 15 stay zero.  k-step s covers dims 16 s + {2 c4,
+      // 2 c4 + 1, + 8, + 9}; for e4m3 dims 64 (s / 4) + 16 c4 + 4 (s % 4) + {0, 1, 2, 3} in the same places
       uint32_t qa[8][4];
       const __nv_bfloat16* qr = a.q + (static_cast<size_t>(c.row) * a.nq + c.kvh * a.group) * 128;
+      float q_exp = 1.0f;                                    // e4m3: power of two that the scores are multiplied with again
 #pragma unroll
       for (int s = 0; s < 8; ++s) {
         const int d0 = KV8 ? 64 * (s >> 2) + 16 * c4 + 4 * (s & 3) : 16 * s + 2 * c4, d1 = KV8 ? d0 + 2 : d0 + 8;
@@ -195,69 +218,90 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
         qa[s][2] = g < a.group ? *reinterpret_cast<const uint32_t*>(qr + g * 128 + d1) : 0u;
         qa[s][3] = 0u;
       }
-      float o[16][4];
+      if constexpr (KV8) {
+        auto vals = [](uint32_t u) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&u)); };
+        float top = 0.f;
 #pragma unroll
-      for (int n = 0; n < 16; ++n)
+        for (int s = 0; s < 8; ++s) {
+          const float2 x = vals(qa[s][0]), y = vals(qa[s][2]);
+          top = fmaxf(top, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(y.x), fabsf(y.y))));
+        }
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+        // the exponent field of the largest moves to 2^14: scale = 2^(14 - e), its inverse goes into the scores
+        const int e = min(max(static_cast<int>(__float_as_uint(top) >> 23) - 127, -100), 100);
+        const float up = __uint_as_float(static_cast<uint32_t>(127 + 14 - e) << 23);
+        q_exp = __uint_as_float(static_cast<uint32_t>(127 - 14 + e) << 23);
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          const float2 x = vals(qa[s][0]), y = vals(qa[s][2]);
+          qa[s][0] = f16x2(x.x * up, x.y * up);
+          qa[s][2] = f16x2(y.x * up, y.y * up);
+        }
+      }
+      // O^T: m-tile n holds 16 dims (rows g, g + 8) by eight heads (columns 2 c4, 2 c4 + 1)
+      float o[8][4];
+#pragma unroll
+      for (int n = 0; n < 8; ++n)
 #pragma unroll
         for (int j = 0; j < 4; ++j) o[n][j] = 0.f;
-      float m = -1e30f, l = 0.f;
-      for (int i = (duo ^ (k0 & 1)); ok && i < c.n; i += 2) {
+      float m = -1e30f, l = 0.f;                             // of head g
+      for (int i = (group - k0) & 3; ok && i < c.n; i += 4) {
         const uint32_t k = k0 + i;
         const int s = k % kS;
         if (!mbar_wait(&full[s], (k / kS) & 1, abort_flag)) { *abort_flag = 1; atomicCAS(a.status, 0, PLOW_ERR_TMA_WAIT | kTagGqa); ok = false; break; }
         const uint8_t* st = ring + s * Cfg::kStageStride;
-        float sc4[2][4];                                     // S of tokens tok0 + 8 t + 2 c4 + {0, 1}, head g in [0], [1]
+        float sc4[4][4];                                     // S of tokens tok0 + 8 t + 2 c4 + {0, 1}, head g in [0], [1]
 #pragma unroll
-        for (int t = 0; t < 2; ++t)
+        for (int t = 0; t < 4; ++t)
 #pragma unroll
           for (int j = 0; j < 4; ++j) sc4[t][j] = 0.f;
         if constexpr (KV8) {
 #pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            const int row = tok0 + 8 * t + g;
+          for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
+            for (int t = 0; t < 4; ++t) {
+              const int row = tok0 + 8 * t + g;
               const uint4 w = *reinterpret_cast<const uint4*>(st + row * 128 + ((4 * h + c4) ^ (row & 7)) * 16);
               const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
               for (int u = 0; u < 4; ++u)
-                mma_bf16(sc4[t], qa[4 * h + u], e4m3_lanes_to_bf16(__byte_perm(ww[u], 0, 0x1404)), e4m3_lanes_to_bf16(__byte_perm(ww[u], 0, 0x3424)));
+                mma_f16(sc4[t], qa[4 * h + u], e4m3x2_to_f16(ww[u]), e4m3x2_to_f16(ww[u] >> 16));
             }
-          }
         } else {
           // 8x8 blocks of an ldmatrix.x4: tokens 8 t .. + 7, dims 16 s .. + 15 and the next 16
           const uint32_t kb = smem_u32(st);
 #pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            const int row = tok0 + 8 * t + (lane & 7);
+          for (int s2 = 0; s2 < 4; ++s2)
 #pragma unroll
-            for (int s2 = 0; s2 < 4; ++s2) {
+            for (int t = 0; t < 4; ++t) {
+              const int row = tok0 + 8 * t + (lane & 7);
               const int chunk = 4 * s2 + (lane >> 3);        // 16-byte chunk of the 256-byte row
               uint32_t b[4];
               ldmatrix4(kb + (chunk >> 3) * 8192 + row * 128 + ((chunk & 7) ^ (row & 7)) * 16, b);
               mma_bf16(sc4[t], qa[2 * s2], b[0], b[1]);
               mma_bf16(sc4[t], qa[2 * s2 + 1], b[2], b[3]);
             }
-          }
         }
-        float vs[4];
+        float vs[8], lv[8];                                  // value scales and their log2
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
+        for (int t = 0; t < 4; ++t) {
           const int tok = tok0 + 8 * t + 2 * c4;
           float f0 = a.scale_log2e, f1 = a.scale_log2e;
           if constexpr (KV8) {
             const float* scs = reinterpret_cast<const float*>(st + 2 * Cfg::kTile);
             const float2 ks = *reinterpret_cast<const float2*>(scs + tok), v2 = *reinterpret_cast<const float2*>(scs + 64 + tok);
-            const float top = a.scale_log2e * 0x1p120f;
-            f0 = fmaxf(fminf(ks.x * top, 3.0e38f), -3.0e38f); f1 = fmaxf(fminf(ks.y * top, 3.0e38f), -3.0e38f);
-            vs[2 * t] = fminf(v2.x * 0x1p60f, 3.0e38f); vs[2 * t + 1] = fminf(v2.y * 0x1p60f, 3.0e38f);
+            const float f = a.scale_log2e * q_exp;
+            f0 = ks.x * f; f1 = ks.y * f;
+            vs[2 * t] = v2.x; vs[2 * t + 1] = v2.y;
+            lv[2 * t] = __log2f(v2.x); lv[2 * t + 1] = __log2f(v2.y);
           }
           sc4[t][0] *= f0; sc4[t][1] *= f1;
         }
         const int t0 = (c.lo_page + c.first + i) * 64 + tok0;
-        if (t0 < c.lo || t0 + 15 > c.hi) {
+        if (t0 < c.lo || t0 + 31 > c.hi) {
 #pragma unroll
-          for (int t = 0; t < 2; ++t)
+          for (int t = 0; t < 4; ++t)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
               const int tok = t0 + 8 * t + 2 * c4 + j;
@@ -265,7 +309,12 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
             }
         }
         // running maximum per head, moved only when exceeded by more than 2^7 (P then stays below that)
-        float mx = fmaxf(fmaxf(sc4[0][0], sc4[0][1]), fmaxf(sc4[1][0], sc4[1][1]));
+        float mx = -INFINITY;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          if constexpr (KV8) mx = fmaxf(mx, fmaxf(sc4[t][0] + lv[2 * t], sc4[t][1] + lv[2 * t + 1]));
+          else mx = fmaxf(mx, fmaxf(sc4[t][0], sc4[t][1]));
+        }
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
         mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
         const bool up = mx > m + 7.0f;
@@ -273,48 +322,55 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
           const float n = up ? mx : m, f = dec_ex2(m - n);
           l *= f;
           m = n;
+          const float f0 = __shfl_sync(0xffffffffu, f, 8 * c4), f1 = __shfl_sync(0xffffffffu, f, 8 * c4 + 4);    // heads 2 c4, 2 c4 + 1
 #pragma unroll
-          for (int j = 0; j < 16; ++j) { o[j][0] *= f; o[j][1] *= f; }
+          for (int j = 0; j < 8; ++j) { o[j][0] *= f0; o[j][1] *= f1; o[j][2] *= f0; o[j][3] *= f1; }
         }
-        // P: the accumulator layout of S is the A layout of the next MMA (k = token)
-        uint32_t pa[4] = {0u, 0u, 0u, 0u};
+        // P: the accumulator layout of S (head g, tokens 2 c4, 2 c4 + 1) is the B layout of the next MMA (column g, k 2 c4, ..)
+        uint32_t pb[4];
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
+        for (int t = 0; t < 4; ++t) {
           float e0 = dec_ex2(sc4[t][0] - m), e1 = dec_ex2(sc4[t][1] - m);
           l += e0 + e1;
-          if constexpr (KV8) { e0 *= vs[2 * t]; e1 *= vs[2 * t + 1]; }
-          const __nv_bfloat162 h0 = __floats2bfloat162_rn(e0, e1);
-          pa[2 * t] = *reinterpret_cast<const uint32_t*>(&h0);
+          if constexpr (KV8) {
+            pb[t] = f16x2(e0 * vs[2 * t], e1 * vs[2 * t + 1]);
+          } else {
+            const __nv_bfloat162 h0 = __floats2bfloat162_rn(e0, e1);
+            pb[t] = *reinterpret_cast<const uint32_t*>(&h0);
+          }
         }
         const uint8_t* vt = st + Cfg::kTile;
-        if constexpr (KV8) {
-          // a lane takes 16 bytes (dims 16 g .. + 15) of the four tokens of its k indices; column g of n-tile n is dim 16 g + n
-          uint32_t w[4][4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int row = tok0 + 2 * c4 + (u & 1) + 8 * (u >> 1);
-            const uint4 x = *reinterpret_cast<const uint4*>(vt + row * 128 + (g ^ (row & 7)) * 16);
-            w[u][0] = x.x; w[u][1] = x.y; w[u][2] = x.z; w[u][3] = x.w;
-          }
+        for (int b16 = 0; b16 < 2; ++b16) {
+          if constexpr (KV8) {
+            // a lane takes 16 bytes (dims 16 g .. + 15) of the four tokens of its k indices; rows g and g + 8 of m-tile n are
+            // dims 16 g + 2 n and 16 g + 2 n + 1
+            uint32_t w[4][4];
 #pragma unroll
-          for (int n = 0; n < 16; ++n) {
-            // byte n of tokens (2 c4, 2 c4 + 1) and (+ 8, + 9) into the high bytes of the two lanes (the low bytes are cut
-            // off by the mask, whatever they hold)
-            const uint32_t sel = ((n & 3) << 4) | ((4 + (n & 3)) << 12);
-            const uint32_t b0 = __byte_perm(w[0][n >> 2], w[1][n >> 2], sel), b1 = __byte_perm(w[2][n >> 2], w[3][n >> 2], sel);
-            mma_bf16(o[n], pa, e4m3_lanes_to_bf16(b0), e4m3_lanes_to_bf16(b1));
-          }
-        } else {
-          const uint32_t vb = smem_u32(vt);
-          const int row = tok0 + (lane & 15);
+            for (int u = 0; u < 4; ++u) {
+              const int row = tok0 + 16 * b16 + 2 * c4 + (u & 1) + 8 * (u >> 1);
+              const uint4 x = *reinterpret_cast<const uint4*>(vt + row * 128 + (g ^ (row & 7)) * 16);
+              w[u][0] = x.x; w[u][1] = x.y; w[u][2] = x.z; w[u][3] = x.w;
+            }
 #pragma unroll
-          for (int n = 0; n < 8; ++n) {
-            // 8x8 blocks: tokens 0 .. 7 and 8 .. 15 of dims 16 n .. + 7, then of dims 16 n + 8 .. + 15
-            const int chunk = 2 * n + (lane >> 4);
-            uint32_t b[4];
-            ldmatrix4_trans(vb + (chunk >> 3) * 8192 + row * 128 + ((chunk & 7) ^ (row & 7)) * 16, b);
-            mma_bf16(o[2 * n], pa, b[0], b[1]);
-            mma_bf16(o[2 * n + 1], pa, b[2], b[3]);
+            for (int n = 0; n < 8; ++n) {
+              // bytes 2 n, 2 n + 1 of tokens 2 c4 and 2 c4 + 1 (then + 8, + 9), side by side per dim
+              const uint32_t sel = n & 1 ? 0x7362 : 0x5140;
+              const uint32_t x = __byte_perm(w[0][n >> 1], w[1][n >> 1], sel), y = __byte_perm(w[2][n >> 1], w[3][n >> 1], sel);
+              const uint32_t va[4] = {e4m3x2_to_f16(x), e4m3x2_to_f16(x >> 16), e4m3x2_to_f16(y), e4m3x2_to_f16(y >> 16)};
+              mma_f16(o[n], va, pb[2 * b16], pb[2 * b16 + 1]);
+            }
+          } else {
+            // 8x8 blocks: tokens 0 .. 7 of dims 16 n .. + 7 and + 8 .. + 15, then tokens 8 .. 15 of the same
+            const uint32_t vb = smem_u32(vt);
+            const int row = tok0 + 16 * b16 + (lane & 7) + 8 * (lane >> 4);
+#pragma unroll
+            for (int n = 0; n < 8; ++n) {
+              const int chunk = 2 * n + ((lane >> 3) & 1);
+              uint32_t va[4];
+              ldmatrix4_trans(vb + (chunk >> 3) * 8192 + row * 128 + ((chunk & 7) ^ (row & 7)) * 16, va);
+              mma_bf16(o[n], va, pb[2 * b16], pb[2 * b16 + 1]);
+            }
           }
         }
         __syncwarp();
@@ -322,62 +378,88 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
       }
       k0 += c.n;
       p += c.n;
-      // ---- the piece is done: merge the eight warps (each holds a partial over its tokens)
+      // ---- the piece is done: this warp's partial (its tokens of the piece) to the merge warps
+      const int buf = n_piece & 1;
+      if (ok && !mbar_wait(&area_free[buf], ((n_piece >> 1) & 1) ^ 1, abort_flag)) { *abort_flag = 1; atomicCAS(a.status, 0, PLOW_ERR_STAGE_WAIT | kTagGqa); ok = false; }
+      if (!ok) break;
+      float* mine = area + (buf * 8 + warp) * a.group * 132;
       l += __shfl_xor_sync(0xffffffffu, l, 1);
       l += __shfl_xor_sync(0xffffffffu, l, 2);
-      if (g < a.group) {
-        float* dst = area + (warp * a.group + g) * 132;
+      if (c4 == 0 && g < a.group) { mine[g * 132 + 128] = m; mine[g * 132 + 129] = l; }
 #pragma unroll
-        for (int n = 0; n < 16; ++n) {
-          // dims of columns 2 c4 and 2 c4 + 1 of n-tile n
-          const int d0 = KV8 ? 32 * c4 + n : 8 * n + 2 * c4, d1 = KV8 ? 32 * c4 + 16 + n : d0 + 1;
-          dst[d0] = o[n][0];
-          dst[d1] = o[n][1];
+      for (int j = 0; j < 2; ++j) {
+        const int head = 2 * c4 + j;
+        if (head < a.group) {
+          float* dst = mine + head * 132;
+#pragma unroll
+          for (int n = 0; n < 8; ++n) {
+            // dims of rows g and g + 8 of m-tile n
+            dst[KV8 ? 16 * g + 2 * n : 16 * n + g] = o[n][j];
+            dst[KV8 ? 16 * g + 2 * n + 1 : 16 * n + 8 + g] = o[n][2 + j];
+          }
         }
-        if (c4 == 0) { dst[128] = m; dst[129] = l; }
       }
-      asm volatile("bar.sync 1, 256;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&area_full[buf]);
+    }
+  } else {
+    // ------------------------------------------------------------------ merge warps
+    // Every warp walks all pieces whatever its waits say (a wait that ran out is carried in `ok`), so the barriers of the
+    // three cannot be left waiting.
+    const int tid = threadIdx.x - 288;
+    bool ok = true;
+    uint32_t n_piece = 0;
+    for (int p = p0; p < p1; ++n_piece) {
+      const Piece c = piece_at(p);
+      const bool is_first = p == p0;
+      p += c.n;
+      const int buf = n_piece & 1;
+      if (ok && !mbar_wait(&area_full[buf], (n_piece >> 1) & 1, abort_flag)) { *abort_flag = 1; atomicCAS(a.status, 0, PLOW_ERR_TMEM_WAIT | kTagGqa); ok = false; }
       const int u0 = prefix[c.row] + c.kvh * c.pages;                              // the line's pages of this (row, kv head)
       const int b0 = static_cast<int>((static_cast<long long>(u0 + 1) * G - 1) / T), b1 = static_cast<int>((static_cast<long long>(u0 + c.pages) * G - 1) / T);
       const bool whole = b0 == b1;
-      const bool is_first = p - c.n == p0;
       float* part = sc.partial + (static_cast<size_t>(blockIdx.x) * 2 + (is_first ? 0 : 1)) * kDecPartial;
       __nv_bfloat16* orow = a.out + (static_cast<size_t>(c.row) * a.nq + c.kvh * a.group) * 128;
-      constexpr float kOut = KV8 ? 0x1p60f : 1.0f;                                // the e4m3 accumulator carries 2^-60
-      for (int e = threadIdx.x; e < a.group * 128; e += 256) {
+      const int stride = a.group * 132;
+      for (int e = tid * 4; ok && e < a.group * 128; e += 384) {                    // four dims of a head
         const int head = e >> 7, d = e & 127;
-        const float* src = area + head * 132;
-        const int stride = a.group * 132;
-        float top = -1e30f;
+        const float* src = area + buf * 8 * stride + head * 132;
+        float top = -1e30f, f[8];
 #pragma unroll
-        for (int w = 0; w < 8; ++w) top = fmaxf(top, src[w * stride + 128]);
-        float acc = 0.f, sum = 0.f;
+        for (int w = 0; w < 8; ++w) { f[w] = src[w * stride + 128]; top = fmaxf(top, f[w]); }
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        float sum = 0.f;
 #pragma unroll
         for (int w = 0; w < 8; ++w) {
-          const float f = dec_ex2(src[w * stride + 128] - top);
-          acc += f * src[w * stride + d];
-          sum += f * src[w * stride + 129];
+          f[w] = dec_ex2(f[w] - top);
+          const float4 x = *reinterpret_cast<const float4*>(src + w * stride + d);
+          acc.x += f[w] * x.x; acc.y += f[w] * x.y; acc.z += f[w] * x.z; acc.w += f[w] * x.w;
+          sum += f[w] * src[w * stride + 129];
         }
-        acc *= kOut;
-        if (whole) orow[e] = __float2bfloat16(sum > 0.f ? acc / sum : 0.f);
-        else {
-          part[e] = acc;
+        if (whole) {
+          const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+          const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x * inv, acc.y * inv), hi = __floats2bfloat162_rn(acc.z * inv, acc.w * inv);
+          *reinterpret_cast<uint2*>(orow + e) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+        } else {
+          part[e] = acc.x; part[e + 1] = acc.y; part[e + 2] = acc.z; part[e + 3] = acc.w;
           if (d == 0) { part[a.group * 128 + head] = top; part[a.group * 129 + head] = sum; }
         }
       }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&area_free[buf]);
       if (!whole) {
         // the CTA that finishes the (row, kv head) last folds the partials of all (in CTA order: the same on every run)
         __threadfence();
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (threadIdx.x == 0) *last_flag = atomicAdd(&sc.arrived[c.row * a.nkv + c.kvh], 1) == b1 - b0;
-        asm volatile("bar.sync 1, 256;" ::: "memory");
+        asm volatile("bar.sync 1, 96;" ::: "memory");
+        if (tid == 0) *last_flag = ok && atomicAdd(&sc.arrived[c.row * a.nkv + c.kvh], 1) == b1 - b0;
+        asm volatile("bar.sync 1, 96;" ::: "memory");
         if (*last_flag) {
           __threadfence();
-          for (int e = threadIdx.x; e < a.group * 128; e += 256) {
+          for (int e = tid; e < a.group * 128; e += 96) {
             const int head = e >> 7;
             auto part_of = [&](int b) {
               const int start = static_cast<int>(static_cast<long long>(T) * b / G);
-              return sc.partial + (static_cast<size_t>(b) * 2 + (start >= u0 ? 0 : (b == b0 ? 1 : 0))) * kDecPartial;
+              return sc.partial + (static_cast<size_t>(b) * 2 + (start >= u0 ? 0 : 1)) * kDecPartial;      // only the first CTA starts before
             };
             float top = -1e30f;
             for (int b = b0; b <= b1; ++b) top = fmaxf(top, __ldcg(part_of(b) + a.group * 128 + head));
@@ -391,8 +473,8 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
             orow[e] = __float2bfloat16(sum > 0.f ? acc / sum : 0.f);
           }
         }
+        asm volatile("bar.sync 1, 96;" ::: "memory");       // the flag is read
       }
-      asm volatile("bar.sync 1, 256;" ::: "memory");        // the merge area is free again
     }
   }
   __syncthreads();

@@ -42,8 +42,7 @@
 namespace plow {
 
 constexpr int kGqaPage = 64;
-constexpr int kGqaThreads = 192;   // TMA warp, MMA warp, 4 softmax warps
-constexpr int kGqaThreads8 = 320;  // + 4 converter warps (e4m3 cache)
+constexpr int kGqaThreads = 192;   // TMA warp, MMA warp, 4 softmax warps (and 4 converter warps for the e4m3 cache)
 constexpr int kGqaRaw = 3;         // raw e4m3 tiles in flight; 4 operand stages behind them
 
 // Rows from which an unsplit bf16 call takes the two-tile kernel of attn_prefill.cu: its items are up to twice as long, so
@@ -85,7 +84,7 @@ template <int HDQ, int HDV, bool KV8 = false> struct GqaCfg {
   // per operand stage: 64 S-column and 64 P-column factors; then a ring of 128 page numbers for the converter warps
   static constexpr int kColBytes = KV8 ? kStages * 128 * 4 + 128 * 4 : 0;
   static constexpr int kSmem = 1024 + kQBytes + kStages * kStageBytes + kRawBytes + kColBytes + 1024;
-  static constexpr int kThreads = KV8 ? kGqaThreads8 : (HDQ == 128 ? kDecThreads : kGqaThreads);
+  static constexpr int kThreads = HDQ == 128 ? kDecThreads : kGqaThreads;     // as many as the decode body has
   static constexpr int kTmemCols = HDV <= 128 ? 256 : 512; // S: 2 x 64, O: HDV
   static_assert(kStages >= 2, "K/V stages do not fit");
   static_assert(kSmem <= 227 * 1024, "shared memory budget");
@@ -328,7 +327,7 @@ gqa_attn_kernel(const GqaArgs a, const __grid_constant__ CUtensorMap tm_q, const
       }
       if (!ok || *abort_flag) { tc_commit(drain_bar); mbar_wait(drain_bar, 0, never_flag); }
     }
-  } else if (KV8 && warp >= 6) {
+  } else if (KV8 && warp >= 6 && warp < 10) {
     // ------------------------------------------------------------------ converter warps (e4m3 cache -> bf16 operand stages)
     // Thread u of the 128 handles work units (row = u % 64, out slab): 64 e4m3 bytes of one token -> 64 bf16 (one
     // 128-byte operand row).  Raw tiles and operand slabs are both 64 rows x 128 bytes with the 128-byte swizzle: the
