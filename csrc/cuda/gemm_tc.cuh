@@ -252,6 +252,13 @@ struct TileSched {
 // silu with the approximate reciprocal (2 ulp): the exact division cost the epilogue warps ~350 clocks per value
 __device__ __forceinline__ float silu_f(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
 
+// acc += v * f for two neighbouring accumulators: one packed instruction (the promotion is bound by issue)
+__device__ __forceinline__ void fma_pair(float& a0, float& a1, uint32_t v0, uint32_t v1, float f0, float f1) {
+  asm("{\n\t.reg .b64 a, v, f;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tmov.b64 f, {%4, %5};\n\t"
+      "fma.rn.f32x2 a, v, f, a;\n\tmov.b64 {%0, %1}, a;\n\t}\n"
+      : "+f"(a0), "+f"(a1) : "r"(v0), "r"(v1), "f"(f0), "f"(f1));
+}
+
 template <int BN, bool FP8, bool DUAL, bool SWAP>
 __global__ void __launch_bounds__((GemmCfg<BN, DUAL, SWAP, FP8>::kThreads), 1)
 gemm_tc_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tm_x,
@@ -479,14 +486,19 @@ gemm_tc_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tm_x,
         // each thread owns one token and needs a single factor.
         constexpr int kNS = SWAP ? (BN + 31) / 32 : 1;
         struct Sc { float sa[kNS]; float wg, wu; };
+        // running pointers: the K block only adds a constant
+        const float* sx_at[kNS];
+#pragma unroll
+        for (int i = 0; i < kNS; ++i)
+          sx_at[i] = a.sx + static_cast<size_t>(t.kb0) * a.ld_sx + min(SWAP ? t.tok0 + i * 32 + lane : tok_i, a.M - 1);
+        const float* wg_at = a.sw + static_cast<size_t>(wblk_g) * KB + t.kb0;
+        const float* wu_at = DUAL ? a.sw + static_cast<size_t>(wblk_u) * KB + t.kb0 : nullptr;
         auto fetch = [&](int kb, Sc& o) {
           if (kb >= KB) return;
-          const float* sxr = a.sx + static_cast<size_t>(kb) * a.ld_sx;
 #pragma unroll
-          for (int i = 0; i < kNS; ++i)
-            o.sa[i] = sxr[min(SWAP ? t.tok0 + i * 32 + lane : tok_i, a.M - 1)];
-          o.wg = a.sw[static_cast<size_t>(wblk_g) * KB + kb];
-          if constexpr (DUAL) o.wu = a.sw[static_cast<size_t>(wblk_u) * KB + kb];
+          for (int i = 0; i < kNS; ++i) { o.sa[i] = *sx_at[i]; sx_at[i] += a.ld_sx; }
+          o.wg = *wg_at++;
+          if constexpr (DUAL) o.wu = *wu_at++;
         };
         float* fw = fac_smem + (warp - 2) * 256;   // [gate BN | up BN] factors of this warp
         Sc s0, s1, s2;
@@ -535,10 +547,8 @@ gemm_tc_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tm_x,
                     const float fs = s0.sa[0] * ((DUAL && col >= kCH) ? s0.wu : s0.wg);
                     f = make_float4(fs, fs, fs, fs);
                   }
-                  acc[col] = fmaf(__uint_as_float(v[q * 16 + j]), f.x, acc[col]);
-                  acc[col + 1] = fmaf(__uint_as_float(v[q * 16 + j + 1]), f.y, acc[col + 1]);
-                  acc[col + 2] = fmaf(__uint_as_float(v[q * 16 + j + 2]), f.z, acc[col + 2]);
-                  acc[col + 3] = fmaf(__uint_as_float(v[q * 16 + j + 3]), f.w, acc[col + 3]);
+                  fma_pair(acc[col], acc[col + 1], v[q * 16 + j], v[q * 16 + j + 1], f.x, f.y);
+                  fma_pair(acc[col + 2], acc[col + 3], v[q * 16 + j + 2], v[q * 16 + j + 3], f.z, f.w);
                 }
               }
             }
