@@ -35,7 +35,7 @@ REGISTRY = [
     KernelSpec("plow_mla_fold", "mla_attention", ("bf16",), dict(v_head=(128,), max_splits=(1, 8)), ("tcgen05", "tmem", "tma")),
     KernelSpec("plow_mla_kv_write", "mla_kv_write", ("e4m3",)),
     KernelSpec("plow_dsa_k_write", "dsa_k_write", ("e4m3",), dict(dim=(128,))),
-    KernelSpec("plow_dsa_select", "dsa_topk", ("e4m3",), dict(heads=(64,), dim=(128,), max_len=(1, 1 << 20)), ("tcgen05", "tmem", "tma"), 26048, 64),
+    KernelSpec("plow_dsa_select", "dsa_topk", ("e4m3",), dict(heads=(64,), dim=(128,), max_len=(1, 1 << 20)), ("tcgen05", "tmem", "tma"), 75776, 128),
     KernelSpec("plow_gdn", "gdn", ("bf16",), dict(head_dim=(128,), conv=(4,))),
     KernelSpec("plow_gated_norm", "gated_norm", ("bf16",)),
     KernelSpec("plow_router_topk", "router_topk", ("f32",), dict(n_experts=(1, 1024))),
