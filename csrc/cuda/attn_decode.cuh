@@ -17,7 +17,7 @@
 //     every bf16 down to 2^-28 of the row's largest exactly; the running maximum is taken of score + log2(value scale), so
 //     P times its value scale stays in f16's range, where it has three more bits than in bf16.  The k index of an MMA may be
 //     any permutation as long as both operands agree, so a lane takes 16 consecutive bytes of a row.
-// 64 sequences of 512 .. 4352 tokens, 32 / 8 heads, with the rotary writer: bf16 117 us (tile form 160 .. 169), e4m3 103 us
+// 64 sequences of 512 .. 4352 tokens, 32 / 8 heads, with the rotary writer: bf16 111 us (tile form 160 .. 169), e4m3 95 us
 // (252 .. 263).  bf16 is at the stream rate; e4m3 is bound by the latency chains of its eight warps.
 // The rates of mma.sync suffice by far (64 of 356 clocks per 16 tokens and SM).
 #pragma once
@@ -33,11 +33,14 @@ constexpr int kDecThreads = 384;          // 8 consumer warps, the producer warp
 constexpr int kDecMaxCtas = 160;
 constexpr int kDecMaxGroup = 8;
 constexpr int kDecMaxRows = 256;
+// Sequences of up to this many pages are not cut when each (row, kv head) can have a CTA of its own: 16 rows x 8 kv heads of 400
+// tokens 16.5 us against 20.6 cut, of 800 tokens 18.5 / 22.6; 4 rows of 1000 tokens, e4m3, 20.6 / 18.5.
+constexpr int kDecUncutPages = 12;
 constexpr int kDecPartial = kDecMaxGroup * 130;      // floats of a partial: [head][128] O, then [head] m, [head] l
 
 // Scratch of a call, in 4-byte words: plan (8), prefix of pages [rows + 1], arrivals [rows * nkv], partials [2 per CTA].
 struct DecScratch {
-  int* plan;            // [0]: 1 = this call is a decode step; [1]: pages
+  int* plan;            // [0]: 1 = this call is a decode step; [1]: pages; [2]: 1 = a CTA per (row, kv head)
   int* prefix;
   int* arrived;
   float* partial;
@@ -45,10 +48,11 @@ struct DecScratch {
     plan = static_cast<int*>(base);
     prefix = plan + 8;
     arrived = prefix + rows + 1;
-    partial = reinterpret_cast<float*>(arrived + rows * nkv);
+    // 16-byte vectors
+    partial = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(arrived + rows * nkv) + 15) & ~static_cast<uintptr_t>(15));
   }
   static int64_t bytes(int rows, int nkv) {
-    return 4ll * (8 + rows + 1 + static_cast<int64_t>(rows) * nkv + 2ll * kDecMaxCtas * kDecPartial);
+    return 4ll * (8 + rows + 1 + static_cast<int64_t>(rows) * nkv + 2ll * kDecMaxCtas * kDecPartial) + 16;
   }
 };
 
@@ -122,7 +126,9 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
   const DecScratch sc(a.scratch, a.rows, a.nkv);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int T = sc.plan[1];
-  const int G = min(static_cast<int>(gridDim.x), T);
+  const bool uncut = sc.plan[2] != 0;
+  // pieces of at least four pages, which is what the warps have in work at a time
+  const int G = uncut ? a.rows * a.nkv : min(static_cast<int>(gridDim.x), (T + 3) / 4);
   if (static_cast<int>(blockIdx.x) >= G) return;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kS; ++s) { mbar_init(&full[s], KV8 ? 33 : 1); mbar_init(&empty[s], 2); }
@@ -132,7 +138,12 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
   }
   for (int i = threadIdx.x; i <= a.rows; i += kDecThreads) prefix[i] = sc.prefix[i];
   __syncthreads();
-  const int p0 = static_cast<int>(static_cast<long long>(T) * blockIdx.x / G), p1 = static_cast<int>(static_cast<long long>(T) * (blockIdx.x + 1) / G);
+  int p0 = static_cast<int>(static_cast<long long>(T) * blockIdx.x / G), p1 = static_cast<int>(static_cast<long long>(T) * (blockIdx.x + 1) / G);
+  if (uncut) {
+    const int row = blockIdx.x / a.nkv, n = (prefix[row + 1] - prefix[row]) / a.nkv;      // 0: an inactive row
+    p0 = prefix[row] + (blockIdx.x % a.nkv) * n;
+    p1 = p0 + n;
+  }
   // the piece that starts at page p of the line: its row, kv head, first page within the sequence's span, length
   struct Piece { int row, kvh, first, n, pages, lo_page, hi, lo; };
   auto piece_at = [&](int p) -> Piece {
@@ -417,7 +428,7 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
       if (ok && !mbar_wait(&area_full[buf], (n_piece >> 1) & 1, abort_flag)) { *abort_flag = 1; atomicCAS(a.status, 0, PLOW_ERR_TMEM_WAIT | kTagGqa); ok = false; }
       const int u0 = prefix[c.row] + c.kvh * c.pages;                              // the line's pages of this (row, kv head)
       const int b0 = static_cast<int>((static_cast<long long>(u0 + 1) * G - 1) / T), b1 = static_cast<int>((static_cast<long long>(u0 + c.pages) * G - 1) / T);
-      const bool whole = b0 == b1;
+      const bool whole = uncut || b0 == b1;
       float* part = sc.partial + (static_cast<size_t>(blockIdx.x) * 2 + (is_first ? 0 : 1)) * kDecPartial;
       __nv_bfloat16* orow = a.out + (static_cast<size_t>(c.row) * a.nq + c.kvh * a.group) * 128;
       const int stride = a.group * 132;
@@ -441,7 +452,7 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
           const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x * inv, acc.y * inv), hi = __floats2bfloat162_rn(acc.z * inv, acc.w * inv);
           *reinterpret_cast<uint2*>(orow + e) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
         } else {
-          part[e] = acc.x; part[e + 1] = acc.y; part[e + 2] = acc.z; part[e + 3] = acc.w;
+          *reinterpret_cast<float4*>(part + e) = acc;
           if (d == 0) { part[a.group * 128 + head] = top; part[a.group * 129 + head] = sum; }
         }
       }
@@ -455,22 +466,40 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
         asm volatile("bar.sync 1, 96;" ::: "memory");
         if (*last_flag) {
           __threadfence();
-          for (int e = tid; e < a.group * 128; e += 96) {
+          // Eight partials' loads at a time (one by one, each waiting for L2, five to seven partials took 25 us).  Only the
+          // first CTA may have started before this (row, kv head), which is then in its second place.
+          const int first_place = static_cast<int>(static_cast<long long>(T) * b0 / G) >= u0 ? 0 : 1;
+          for (int e = tid * 4; e < a.group * 128; e += 384) {
             const int head = e >> 7;
-            auto part_of = [&](int b) {
-              const int start = static_cast<int>(static_cast<long long>(T) * b / G);
-              return sc.partial + (static_cast<size_t>(b) * 2 + (start >= u0 ? 0 : 1)) * kDecPartial;      // only the first CTA starts before
-            };
-            float top = -1e30f;
-            for (int b = b0; b <= b1; ++b) top = fmaxf(top, __ldcg(part_of(b) + a.group * 128 + head));
-            float acc = 0.f, sum = 0.f;
-            for (int b = b0; b <= b1; ++b) {
-              const float* q = part_of(b);
-              const float f = dec_ex2(__ldcg(q + a.group * 128 + head) - top);
-              acc += f * __ldcg(q + e);
-              sum += f * __ldcg(q + a.group * 129 + head);
+            float top = -1e30f, sum = 0.f;
+            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int b = b0; b <= b1; b += 8) {
+              float m[8], l[8];
+              float4 x[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const float* q = sc.partial + (static_cast<size_t>(b + j) * 2 + (b + j == b0 ? first_place : 0)) * kDecPartial;
+                const bool in = b + j <= b1;
+                m[j] = in ? __ldcg(q + a.group * 128 + head) : -1e30f;
+                l[j] = in ? __ldcg(q + a.group * 129 + head) : 0.f;
+                x[j] = in ? __ldcg(reinterpret_cast<const float4*>(q + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
+              }
+              float t = top;
+#pragma unroll
+              for (int j = 0; j < 8; ++j) t = fmaxf(t, m[j]);
+              const float f0 = dec_ex2(top - t);
+              top = t;
+              acc.x *= f0; acc.y *= f0; acc.z *= f0; acc.w *= f0; sum *= f0;
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                const float f = dec_ex2(m[j] - t);
+                acc.x += f * x[j].x; acc.y += f * x[j].y; acc.z += f * x[j].z; acc.w += f * x[j].w;
+                sum += f * l[j];
+              }
             }
-            orow[e] = __float2bfloat16(sum > 0.f ? acc / sum : 0.f);
+            const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(acc.x * inv, acc.y * inv), hi = __floats2bfloat162_rn(acc.z * inv, acc.w * inv);
+            *reinterpret_cast<uint2*>(orow + e) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
           }
         }
         asm volatile("bar.sync 1, 96;" ::: "memory");       // the flag is read

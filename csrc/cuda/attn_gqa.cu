@@ -124,7 +124,7 @@ __global__ void gqa_build_items(const int* seq, const int* pos, int rows, int tq
 // step as one line for attn_decode.cuh; otherwise the items of the tile kernel as above.
 __global__ void __launch_bounds__(kDecMaxRows)
 gqa_plan_small(const int* seq, const int* pos, int rows, int tq, int nkv, int window, int tiles_per_split, int max_splits, GqaItem* items,
-               int* n_items, int* row_ns, int cap, void* dec, int* status) {
+               int* n_items, int* row_ns, int cap, void* dec, int grid, int* status) {
   plow::pdl_launch_dependents();
   plow::pdl_wait();
   __shared__ int warp_sum[kDecMaxRows / 32], n_sh;
@@ -145,7 +145,9 @@ gqa_plan_small(const int* seq, const int* pos, int rows, int tq, int nkv, int wi
     int base = 0, total = 0;
     for (int w = 0; w < kDecMaxRows / 32; ++w) { if (w < warp) base += warp_sum[w]; total += warp_sum[w]; }
     if (r < rows) sc.prefix[r] = base + incl - n;
-    if (r == 0) { sc.plan[0] = 1; sc.plan[1] = total; sc.prefix[rows] = total; *n_items = 0; }
+    // few short sequences: whole ones per CTA, nothing to fold
+    const bool uncut = !__syncthreads_or(n > kDecUncutPages * nkv) && rows * nkv <= grid;
+    if (r == 0) { sc.plan[0] = 1; sc.plan[1] = total; sc.plan[2] = uncut; sc.prefix[rows] = total; *n_items = 0; }
     for (int i = r; i < rows * nkv; i += kDecMaxRows) sc.arrived[i] = 0;
     if (r < rows) row_ns[r] = live ? 1 : 0;
     return;
@@ -890,9 +892,11 @@ int plow_gqa_attention(const void* q, const void* kc, const void* vc, int64_t n_
   }
   // small calls: the plan kernel finds out on the device whether this is a decode step
   if (rows > kDecMaxRows || hd != 128 || group > kDecMaxGroup) dec = nullptr;
+  int grid = sm_count();
+  if (dec && grid > kDecMaxCtas) grid = kDecMaxCtas;
   if (dec) {
     plow::launch_serial(gqa_plan_small, dim3(1), dim3(kDecMaxRows), 0, stream, seq, pos, rows, tq, nkv, window, tiles_per_split, max_splits,
-                        static_cast<GqaItem*>(items), n_items, row_ns, item_cap, dec, status);
+                        static_cast<GqaItem*>(items), n_items, row_ns, item_cap, dec, grid, status);
   } else {
     cudaMemsetAsync(n_items, 0, sizeof(int), stream);
     plow::launch_serial(gqa_build_items, dim3((rows + 255) / 256), dim3(256), 0, stream, seq, pos, rows, tq, nkv, window, tiles_per_split, max_splits,
@@ -905,8 +909,6 @@ int plow_gqa_attention(const void* q, const void* kc, const void* vc, int64_t n_
   a.rows = rows; a.nq = nq; a.nkv = nkv; a.group = group; a.max_pages = max_pages; a.max_splits = max_splits; a.window = window;
   a.scale_log2e = softmax_scale * 1.4426950408889634f;
   a.kv_scale = kv_scale;
-  int grid = sm_count();
-  if (dec && grid > kDecMaxCtas) grid = kDecMaxCtas;
   if (!dec && item_cap < grid) grid = item_cap;
   int r = kv_scale ? launch_gqa8<128>(a, q, kc, vc, n_pages, grid, stream)
           : hd == 128 ? launch_gqa<128>(a, q, kc, vc, n_pages, grid, stream) : launch_gqa<256>(a, q, kc, vc, n_pages, grid, stream);

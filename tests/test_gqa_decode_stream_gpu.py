@@ -33,7 +33,9 @@ def _case(lens, nq, nkv, kv8, seed, idle=()):
 @pytest.mark.parametrize("lens,nq,nkv,window,idle", [
     ([1], 32, 8, 0, ()), ([1, 2, 63, 64, 65, 127, 128, 129], 8, 8, 0, (3,)), ([5000], 32, 8, 0, ()), ([4000, 1, 1, 17], 8, 1, 0, (0, 2)),
     ([100 + 37 * i for i in range(64)], 32, 8, 0, (0, 31, 63)), ([3000, 700, 70], 16, 4, 200, ()), ([513] * 256, 4, 2, 0, ()),
-    ([1200, 800], 8, 4, 64, ()), ([40, 40, 40], 32, 8, 0, (0, 1, 2))])
+    ([1200, 800], 8, 4, 64, ()), ([40, 40, 40], 32, 8, 0, (0, 1, 2)),
+    # whole sequences per CTA up to their longest, and one page or one row too many; a fold of more partials than one batch
+    ([768] * 18, 32, 8, 0, (5,)), ([768] * 19, 32, 8, 0, ()), ([768, 769], 32, 8, 0, ()), ([9000], 8, 1, 0, ())])
 def test_decode_stream(lens, nq, nkv, window, idle, kv8):
     from plow_b200.ops import gqa, native
     q, kc, vc, pt, seq, pos, ks, kd, vd = _case(lens, nq, nkv, kv8, len(lens) + sum(lens) % 97, idle)
