@@ -67,10 +67,12 @@ struct MlaArgs {
 // ---------------------------------------------------------------------------------------------
 constexpr int kMlaClaimSlots = 256;   // one work counter per launch between two builds of the list (layers of a step)
 
-__global__ void mla_build_items(const int* kvlen, int T, int tiles_per_split, int max_splits,
-                                MlaItem* items, int* n_items, int* claims) {
-  // one thread per request: split count and tiles per split, then its offset in the list.  Up to 256 requests the
-  // list is ordered by decreasing tiles per item (longest first), which together with the dynamic hand-out in the
+// 64 requests of up to nine splits: 10.5 us with a thread per request (its whole list of items, and the sums before it, in series).
+constexpr int kMlaItemThreads = 1024;
+
+__global__ void __launch_bounds__(kMlaItemThreads)
+mla_build_items(const int* kvlen, int T, int tiles_per_split, int max_splits, MlaItem* items, int* n_items, int* claims) {
+  // split count and tiles per split of every request, then its offset in the list.  Up to 256 requests the list is ordered by decreasing tiles per item (longest first), which together with the dynamic hand-out in the
   // attention kernel keeps the last CTAs from finishing long after the rest; larger batches keep request order.
   extern __shared__ int cnt[];     // [T] splits, then [T] tiles per split
   int* pers = cnt + T;
@@ -84,27 +86,29 @@ __global__ void mla_build_items(const int* kvlen, int T, int tiles_per_split, in
     pers[r] = tiles > 0 ? per : 0;
   }
   __syncthreads();
+  // a warp per request: its lanes sum the splits of the requests before it, then write its items
   const bool by_size = T <= 256;
-  for (int r = threadIdx.x; r < T; r += blockDim.x) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int r = warp; r < T; r += blockDim.x >> 5) {
     const int my = pers[r];
-    int off = 0;
-    for (int q = 0; q < T; ++q) {
+    int off = 0, tot = 0;
+    for (int q = lane; q < T; q += 32) {
+      const int c = cnt[q];
       const bool before = by_size ? (pers[q] > my || (pers[q] == my && q < r)) : q < r;
-      off += before ? cnt[q] : 0;
+      off += before ? c : 0;
+      tot += c;
+    }
+    off = __reduce_add_sync(0xffffffffu, off);
+    if (r == 0) {
+      tot = __reduce_add_sync(0xffffffffu, tot);
+      if (lane == 0) *n_items = 2 * tot;
     }
     const int tiles = (kvlen[r] + kMlaPage - 1) / kMlaPage;
     const int ns = cnt[r], per = my > 0 ? my : 1;
-    for (int split = 0; split < ns; ++split) {
-      const int t0 = split * per;
-      const int nt = min(per, tiles - t0);
-      items[2 * (off + split)] = MlaItem{r, 0, split, t0, nt, 0, 0, 0};
-      items[2 * (off + split) + 1] = MlaItem{r, 1, split, t0, nt, 0, 0, 0};
+    for (int i = lane; i < 2 * ns; i += 32) {
+      const int split = i >> 1, t0 = split * per;
+      items[2 * off + i] = MlaItem{r, i & 1, split, t0, min(per, tiles - t0), 0, 0, 0};
     }
-  }
-  if (threadIdx.x == 0) {
-    int tot = 0;
-    for (int q = 0; q < T; ++q) tot += cnt[q];
-    *n_items = 2 * tot;
   }
 }
 
@@ -532,7 +536,7 @@ void plow_mla_set_trace(void* p) { g_mla_trace = static_cast<long long*>(p); }
 int plow_mla_build_items(const int* kvlen, int T, int tiles_per_split, int max_splits, void* items, int* n_items, int* claims, void* stream_) {
   using namespace plow;
   if (T <= 0 || max_splits <= 0 || tiles_per_split <= 0) return -1;
-  cudaError_t e = launch_serial(mla_build_items, dim3(1), dim3(256), 2 * T * sizeof(int), reinterpret_cast<cudaStream_t>(stream_),
+  cudaError_t e = launch_serial(mla_build_items, dim3(1), dim3(kMlaItemThreads), 2 * T * sizeof(int), reinterpret_cast<cudaStream_t>(stream_),
                              kvlen, T, tiles_per_split, max_splits, static_cast<MlaItem*>(items), n_items, claims);
   if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 4000 + static_cast<int>(e);
@@ -560,7 +564,7 @@ int plow_mla_decode(const void* q8, const float* sq, const void* kv, const float
   static DeviceOnce attr;
   if (ensure_smem(attr, mla_decode_kernel, kMlaSmem) != cudaSuccess) return 3000;
   if (build_items)
-    launch_serial(mla_build_items, dim3(1), dim3(256), 2 * T * sizeof(int), stream, kvlen, T, tiles_per_split, max_splits,
+    launch_serial(mla_build_items, dim3(1), dim3(kMlaItemThreads), 2 * T * sizeof(int), stream, kvlen, T, tiles_per_split, max_splits,
                   static_cast<MlaItem*>(items), n_items, claims);
   MlaArgs a;
   a.q8 = static_cast<const uint8_t*>(q8); a.sq = sq; a.kv_scale = kv_scale; a.kv_smax = kv_smax; a.page_table = page_table; a.slot_of = slot_of; a.kvlen = kvlen;

@@ -169,7 +169,14 @@ struct FoldArgs {
   int T, heads, max_splits, tiles_per_split, ld_saq;
 };
 
-__global__ void __launch_bounds__(kProjThreads, 1)
+// Merge of the splits, then the product with W_uv, for 128 tokens of one head.  The merge waits for L2: 64 tokens of up to nine splits
+// are 0.5 MB per CTA and phase (the product's two halves of the latent).  Eight warps merge, four of them read the result back; with four
+// merge warps, which started a phase's loads only when the tensor core had read the last one's operand, 64 sequences of 1024 ..
+// 8192 tokens took 23 us.
+constexpr int kFoldWarps = 8;
+constexpr int kFoldThreads = 32 + 32 * kFoldWarps;
+
+__global__ void __launch_bounds__(kFoldThreads, 1)
 mla_fold_kernel(const FoldArgs a, const __grid_constant__ CUtensorMap tm_w) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -184,7 +191,7 @@ mla_fold_kernel(const FoldArgs a, const __grid_constant__ CUtensorMap tm_w) {
   const int h = blockIdx.x, t0 = blockIdx.y * 128;
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
-    mbar_init(b_full, 1); mbar_init(a_ready, 4); mbar_init(&done[0], 1); mbar_init(&done[1], 1);
+    mbar_init(b_full, 1); mbar_init(a_ready, kFoldWarps); mbar_init(&done[0], 1); mbar_init(&done[1], 1);
     *abort_flag = 0; fence_mbar_init();
   }
   if (warp == 0) { tmem_alloc(holder, 128); tmem_relinquish(); }
@@ -211,16 +218,17 @@ mla_fold_kernel(const FoldArgs a, const __grid_constant__ CUtensorMap tm_w) {
       }
     }
   } else {
+    const int mw = warp - 1;                       // merge warp
     const int lq = warp & 3;
     const int li = lq * 32 + lane;
     const int t = t0 + li;
-    const bool live = t < a.T;
+    const bool live = t < a.T && mw < 4;           // warps 1 .. 4 hold a token per lane
     const uint32_t lane_addr = static_cast<uint32_t>(lq * 32) << 16;
     pdl_wait();      // partials and log-sum-exps come from the attention kernel (warp 0 only touches W_uv, a weight)
     // merge weights of this (token, head), shared with the other merge warps through shared memory
     float* wsm = reinterpret_cast<float*>(smem + 131072 + 256);       // [128 rows][kFoldSplits]
     int* nsm = reinterpret_cast<int*>(wsm + 128 * kFoldSplits);       // [128 rows]
-    {
+    if (mw < 4) {
       float wgt[kFoldSplits];
 #pragma unroll
       for (int s = 0; s < kFoldSplits; ++s) wgt[s] = 0.f;
@@ -247,24 +255,23 @@ mla_fold_kernel(const FoldArgs a, const __grid_constant__ CUtensorMap tm_w) {
       for (int s = 0; s < kFoldSplits; ++s) wsm[li * kFoldSplits + s] = wgt[s];
       nsm[li] = ns;
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * kFoldWarps) : "memory");
     const int n_live = min(128, a.T - t0);
     bool ok = true;
     for (int p = 0; p < 2 && ok; ++p) {
-      if (p == 1 && !mbar_wait(&done[0], 0, abort_flag)) { *abort_flag = 1; atomicCAS(a.status, 0, PLOW_ERR_TMEM_WAIT | kTagMlaProj); ok = false; break; }
-      // A operand: warp w fills rows w, w+4, w+8, ... (so the live rows are spread over all four warps), eight
+      // A operand: merge warp w fills rows w, w+8, w+16, ... (so the live rows are spread over all the warps), eight
       // rows at a time.  For one row the 32 lanes fetch the row's 256 latent columns of this phase as one
       // coalesced 512-byte read per split (lane = 16-byte unit); the eight rows' loads of a split are issued
       // together, so a batch costs one memory round trip per split.  The merged unit goes to its swizzled
       // place: unit u of chunk c at (u ^ (row & 7)) * 16.
-      for (int kb = 0; kb < 32; kb += 8) {
-        if (lq + 4 * kb >= n_live) break;          // rows ascend: nothing live further on (warp-uniform)
+      for (int kb = 0; kb < 128 / kFoldWarps; kb += 8) {
+        if (kb > 0 && mw + kFoldWarps * kb >= n_live) break;          // rows ascend: nothing live further on (warp-uniform)
         float acc[8][8];
         int nsr[8];
         int ns_b = 0;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int row = lq + 4 * (kb + i);
+          const int row = mw + kFoldWarps * (kb + i);
           nsr[i] = row < n_live ? nsm[row] : 0;
           ns_b = max(ns_b, nsr[i]);
 #pragma unroll
@@ -274,23 +281,25 @@ mla_fold_kernel(const FoldArgs a, const __grid_constant__ CUtensorMap tm_w) {
           uint4 v[8];
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            const int row = lq + 4 * (kb + i);
+            const int row = mw + kFoldWarps * (kb + i);
             v[i] = make_uint4(0u, 0u, 0u, 0u);
             if (sp < nsr[i])
               v[i] = *reinterpret_cast<const uint4*>(a.opart + ((static_cast<size_t>(t0 + row) * a.max_splits + sp) * a.heads + h) * 512 + p * 256 + lane * 8);
           }
 #pragma unroll
           for (int i = 0; i < 8; ++i) {
-            const int row = lq + 4 * (kb + i);
+            const int row = mw + kFoldWarps * (kb + i);
             const float wv = wsm[(row & 127) * kFoldSplits + sp];
             const __nv_bfloat162* hh = reinterpret_cast<const __nv_bfloat162*>(&v[i]);
 #pragma unroll
             for (int j = 0; j < 4; ++j) { const float2 f = __bfloat1622float2(hh[j]); acc[i][2 * j] += wv * f.x; acc[i][2 * j + 1] += wv * f.y; }
           }
         }
+        // the tensor core has read the last phase's operand
+        if (p == 1 && kb == 0 && !mbar_wait(&done[0], 0, abort_flag)) { *abort_flag = 1; atomicCAS(a.status, 0, PLOW_ERR_TMEM_WAIT | kTagMlaProj); ok = false; break; }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          const int row = lq + 4 * (kb + i);
+          const int row = mw + kFoldWarps * (kb + i);
           uint4 o;
           __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
@@ -299,11 +308,14 @@ mla_fold_kernel(const FoldArgs a, const __grid_constant__ CUtensorMap tm_w) {
           *reinterpret_cast<uint4*>(sa + c * 16384 + row * 128 + ((uu ^ (row & 7)) << 4)) = o;
         }
       }
+      if (!ok) break;
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(a_ready);
     }
-    if (ok && mbar_wait(&done[1], 0, abort_flag)) {
+    if (mw >= 4) {
+      // the result is read back by warps 1 .. 4
+    } else if (ok && mbar_wait(&done[1], 0, abort_flag)) {
       tc_fence_after();
       float r[128];
       float amax = 0.f;
@@ -391,7 +403,7 @@ int plow_mla_fold(const void* opart, const float* lse, const int* kvlen, const v
   a.opart = static_cast<const __nv_bfloat16*>(opart); a.lse = lse; a.kvlen = kvlen; a.ao = static_cast<__nv_bfloat16*>(ao);
   a.aq = static_cast<uint8_t*>(aq); a.saq = saq; a.status = status; a.T = T; a.heads = heads; a.max_splits = max_splits;
   a.tiles_per_split = tiles_per_split; a.ld_saq = ld_saq;
-  cudaError_t e = launch_serial(mla_fold_kernel, dim3(heads, (T + 127) / 128), dim3(kProjThreads), smem,
+  cudaError_t e = launch_serial(mla_fold_kernel, dim3(heads, (T + 127) / 128), dim3(kFoldThreads), smem,
                              reinterpret_cast<cudaStream_t>(stream_), a, tw);
   if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 4000 + static_cast<int>(e);
