@@ -79,7 +79,7 @@ def chunked_prefill(qkvz, ba, conv_w, a_log, dt_bias, conv_hist, S, hk, hv, d=12
     K^[j] = exp(g_C - g_j) k_j, so M_c and B_c of every chunk are formed in parallel and only  S <- S M_c + B_c  runs in
     sequence (one batched matrix product per chunk).  Outputs:  O = diag(gamma) Q S0^T + tril(Q K^T (.) exp(g_i - g_j)) U.
     Everything is f32 batched matrix algebra (cuBLAS / cuSOLVER through PyTorch: library GEMMs, not a hand-written
-    kernel); the token-by-token kernel (csrc/cuda/gdn.cu) keeps decode and short runs.  Padding rows of the last chunk
+    kernel); the recurrence kernel (csrc/cuda/gdn.cu) keeps decode and short runs.  Padding rows of the last chunk
     carry beta = 0, log-decay 0 and zero keys, which leaves the state untouched.
 
     qkvz [T, C + hv d] bf16, ba [T, 2 hv]; conv_hist [C, conv - 1] and S [hv, d, d] f32 are the sequence's state before

@@ -193,7 +193,7 @@ def profile_summary() -> list:
         e[1] += a.elapsed_time(b)
     PROFILE.clear()
     return sorted(((k, c, t) for k, (c, t) in agg.items()), key=lambda x: -x[2])
-_KERNELS_PER_CALL = {"plow_gqa_attention": 2, "plow_dsa_select": 3, "plow_mla_prefill_attention": 3, "plow_gdn": 2}
+_KERNELS_PER_CALL = {"plow_gqa_attention": 2, "plow_dsa_select": 3, "plow_mla_prefill_attention": 2, "plow_gdn": 2}
 
 
 def call(name: str, *args) -> None:

@@ -1,4 +1,4 @@
-"""Device sampler (csrc/cuda/sampler.cu): temperature / top-k / top-p / min-p and the draw, one CTA per row."""
+"""Device sampler (csrc/cuda/sampler.cu): temperature / top-k / top-p / min-p and the draw, one cluster of CTAs per row."""
 from __future__ import annotations
 
 import torch

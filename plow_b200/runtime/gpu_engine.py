@@ -550,7 +550,7 @@ class GpuEngine(EngineBase):
                     gathered=False)
 
     # Runs of at least this many new rows take the chunked gated-delta-rule prefill (0 = off, the default: that path is
-    # batched matrix algebra through cuBLAS / cuSOLVER, and the serving default keeps the hand-written token-by-token
+    # batched matrix algebra through cuBLAS / cuSOLVER, and the serving default keeps the hand-written recurrence
     # kernel on this op; set PLOW_GDN_CHUNKED_MIN_RUN=128 to trade that for a several times faster long-prompt prefill).
     GDN_CHUNKED_MIN_RUN = int(os.environ.get("PLOW_GDN_CHUNKED_MIN_RUN", "0"))
 
@@ -761,7 +761,7 @@ class GpuEngine(EngineBase):
             gdn_ops.gdn(qkvz, ba, conv_w, a_log, dt_bias, conv_state, ssm_state, self.d_in[1], self.d_in[2], hk, hv, hd, conv, out=out)
             return
         # long runs of new rows: chunked (WY-form) prefill, 64 tokens at a time (ops/gdn.py::chunked_prefill); everything
-        # else (decode riders, short runs, padding rows) stays on the token-by-token kernel, one call per row range
+        # else (decode riders, short runs, padding rows) stays on the recurrence kernel, one call per row range
         for slot, r0, r1, fresh in plan["chunked"]:
             hist = torch.zeros_like(conv_state[slot], dtype=F32) if fresh else conv_state[slot]
             S0 = torch.zeros_like(ssm_state[slot], dtype=F32) if fresh else ssm_state[slot]
