@@ -15,8 +15,10 @@
 //   * e4m3 elements become f16 in registers, one conversion per pair (as bf16, by integer instructions, a pair took four and
 //     the ALU pipe half the time); key scales multiply S, value scales P.  Q is scaled by a power of two into f16, which holds
 //     every bf16 down to 2^-28 of the row's largest exactly; the running maximum is taken of score + log2(value scale), so
-//     P times its value scale stays in f16's range, where it has three more bits than in bf16.  The k index of an MMA may be
-//     any permutation as long as both operands agree, so a lane takes 16 consecutive bytes of a row.
+//     P times its value scale stays in f16's range.  There it has three more bits than in bf16 down to 2^-17 of the largest weight
+//     of the warp, fewer below, and none below 2^-25: errors against 64 bits are the same or smaller up to 131072 tokens.  Cells that
+//     no row sees may hold anything: their scores, value scales and value bytes are replaced on the pages that lo or hi cuts.  The
+//     k index of an MMA may be any permutation as long as both operands agree, so a lane takes 16 consecutive bytes of a row.
 // 64 sequences of 512 .. 4352 tokens, 32 / 8 heads, with the rotary writer: bf16 111 us (tile form 160 .. 169), e4m3 95 us
 // (252 .. 263).  bf16 is at the stream rate; e4m3 is bound by the latency chains of its eight warps.
 // The rates of mma.sync suffice by far (64 of 356 clocks per 16 tokens and SM).
@@ -305,18 +307,23 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
             const float f = a.scale_log2e * q_exp;
             f0 = ks.x * f; f1 = ks.y * f;
             vs[2 * t] = v2.x; vs[2 * t + 1] = v2.y;
-            lv[2 * t] = __log2f(v2.x); lv[2 * t + 1] = __log2f(v2.y);
+            // a value scale of zero weighs nothing; the bound keeps exponentials over such tokens alone finite
+            lv[2 * t] = fmaxf(__log2f(fabsf(v2.x)), -96.0f); lv[2 * t + 1] = fmaxf(__log2f(fabsf(v2.y)), -96.0f);
           }
           sc4[t][0] *= f0; sc4[t][1] *= f1;
         }
         const int t0 = (c.lo_page + c.first + i) * 64 + tok0;
-        if (t0 < c.lo || t0 + 31 > c.hi) {
+        const bool edge = t0 < c.lo || t0 + 31 > c.hi;       // some of the 32 tokens are hidden
+        if (edge) {
 #pragma unroll
           for (int t = 0; t < 4; ++t)
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
               const int tok = t0 + 8 * t + 2 * c4 + j;
-              if (tok < c.lo || tok > c.hi) sc4[t][j] = -INFINITY;
+              if (tok < c.lo || tok > c.hi) {
+                sc4[t][j] = -INFINITY;
+                if constexpr (KV8) vs[2 * t + j] = 0.f;      // the cell may hold anything
+              }
             }
         }
         // running maximum per head, moved only when exceeded by more than 2^7 (P then stays below that)
@@ -362,6 +369,13 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
               const int row = tok0 + 16 * b16 + 2 * c4 + (u & 1) + 8 * (u >> 1);
               const uint4 x = *reinterpret_cast<const uint4*>(vt + row * 128 + (g ^ (row & 7)) * 16);
               w[u][0] = x.x; w[u][1] = x.y; w[u][2] = x.z; w[u][3] = x.w;
+            }
+            if (edge) {                                      // NaN codes of hidden tokens would survive the weight zero
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                const int tok = t0 + 16 * b16 + 2 * c4 + (u & 1) + 8 * (u >> 1);
+                if (tok < c.lo || tok > c.hi) w[u][0] = w[u][1] = w[u][2] = w[u][3] = 0u;
+              }
             }
 #pragma unroll
             for (int n = 0; n < 8; ++n) {

@@ -70,3 +70,57 @@ def test_decode_workspace_serves_fewer_rows_and_other_calls():
         ref = gqa.reference(q, kc, vc, pt, cs, cp)
         assert (out.float() - ref).norm() / ref.norm() < 6e-3
     native.check_status()
+
+
+@pytest.mark.parametrize("form", ["stream", "tile"])
+@pytest.mark.parametrize("lens,nq,nkv,window", [([1, 63, 64, 65, 130, 700], 32, 8, 0), ([900, 77, 3000, 40], 8, 4, 70), ([5, 1500], 16, 2, 33)])
+def test_unused_e4m3_cells_may_hold_anything(lens, nq, nkv, window, form):
+    """Cells that no row attends to (behind a sequence's end, before its window) are NaN codes with NaN and infinite scales."""
+    from plow_b200.ops import gqa, native
+    q, kc, vc, pt, seq, pos, ks, kd, vd = _case(lens, nq, nkv, True, sum(lens))
+    if form == "tile":                                        # two tokens of a sequence in a row: no decode step
+        n = torch.tensor([0 if v == 1 else 1 for v in lens], device="cuda").bool()
+        seq, pos = seq.repeat_interleave(2), torch.stack([torch.where(n, pos - 1, -1), pos], 1).view(-1).int().contiguous()
+        q = q.repeat_interleave(2, 0).contiguous()
+    rows = len(pos)
+    ref = gqa.reference(q, kd, vd, pt, seq, pos, window=window)
+    used = torch.zeros(kc.shape[0], 64, dtype=torch.bool, device="cuda")
+    for r in range(rows):
+        hi = int(pos[r])
+        t = torch.arange(max(0, hi - window + 1) if window else 0, hi + 1, device="cuda")
+        used[pt[int(seq[r])][t // 64].long(), t % 64] = True
+    kc, vc, ks = kc.view(torch.uint8).clone(), vc.view(torch.uint8).clone(), ks.clone()
+    kc[~used] = 0x7F
+    vc[~used] = 0xFF
+    bad = torch.full_like(ks, float("nan"))
+    bad[:, 1::2] = float("inf")
+    ks = torch.where(used[..., None], ks, bad)
+    ws = gqa.AttnWorkspace(rows, nq, nkv, 128, max(lens), "cuda")
+    out = gqa.attention(q, kc, vc, pt, seq, pos, ws, window=window, kv_scale=ks)
+    torch.cuda.synchronize()
+    native.check_status()
+    live = pos >= 0
+    assert (out[live].float() - ref[live]).norm() / ref[live].norm() < 6e-3
+
+
+@pytest.mark.parametrize("form", ["stream", "tile"])
+@pytest.mark.parametrize("zero", ["some", "pages", "all"])
+def test_zero_value_scales(zero, form):
+    """A value scale of zero is a value of zero: the token keeps its share of the softmax."""
+    from plow_b200.ops import gqa, native
+    lens, nq, nkv = [70, 500, 1300], 8, 2
+    q, kc, vc, pt, seq, pos, ks, kd, vd = _case(lens, nq, nkv, True, 11)
+    if form == "tile":
+        seq, pos, q = seq.repeat_interleave(2), torch.stack([pos - 1, pos], 1).view(-1).contiguous(), q.repeat_interleave(2, 0).contiguous()
+    t = torch.arange(64, device="cuda")
+    hide = {"some": (t % 3 == 0)[None].repeat(kc.shape[0], 1), "pages": (torch.arange(kc.shape[0], device="cuda") % 2 == 0)[:, None].repeat(1, 64),
+            "all": torch.ones(kc.shape[0], 64, dtype=torch.bool, device="cuda")}[zero]
+    ks = ks.clone()
+    ks[..., nkv:][hide] = 0.0
+    vd = torch.where(hide[..., None, None], torch.zeros_like(vd), vd)
+    ref = gqa.reference(q, kd, vd, pt, seq, pos)
+    ws = gqa.AttnWorkspace(len(pos), nq, nkv, 128, max(lens), "cuda")
+    out = gqa.attention(q, kc, vc, pt, seq, pos, ws, kv_scale=ks).float()
+    torch.cuda.synchronize()
+    native.check_status()
+    assert (out - ref).norm() <= 6e-3 * ref.norm()            # "all": exactly zero
