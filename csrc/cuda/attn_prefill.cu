@@ -140,10 +140,14 @@ __device__ __forceinline__ float ex2(float x) { float r; asm("ex2.approx.ftz.f32
 
 // 2^x of two values on the FMA pipe: x = n + f with n the nearest integer (the bits of x + 1.5 * 2^23 hold it), a degree-5
 // minimax polynomial of 2^f on [-1/2, 1/2] (Remez fit; with its f32 roundings off by 2.1e-7 at most, 8e-8 rms, the same
-// as ex2.approx), and n added to the exponent.  x <= 127; below -126 the result stays at 2^-126.
+// as ex2.approx), and n added to the exponent.  x <= 127; from -127 down (masked keys) the result is the smallest denormal, which is
+// zero as a bf16.  A NaN comes out as the largest finite number, infinite as a bf16: a row's sum beyond kNanSum tells that it holds one
+// (honest ones stay below 2^7 times the number of keys).
+constexpr float kNanSum = 0x1p100f;
+__device__ __forceinline__ float max_nan(float a, float b) { float r; asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b)); return r; }
 __device__ __forceinline__ void ex2_fma(float x0, float x1, float& r0, float& r1) {
   const f32x2 magic = pack2(12582912.0f, 12582912.0f), unmagic = pack2(-12582912.0f, -12582912.0f);
-  const f32x2 x = pack2(fmaxf(x0, -126.0f), fmaxf(x1, -126.0f));
+  const f32x2 x = pack2(max_nan(x0, -127.0f), max_nan(x1, -127.0f));
   const f32x2 t = add2(x, magic);
   const f32x2 f = fma2(add2(t, unmagic), pack2(-1.0f, -1.0f), x);
   f32x2 p = fma2(pack2(0.0013276472454890609f, 0.0013276472454890609f), f, pack2(0.009675540961325169f, 0.009675540961325169f));
@@ -453,10 +457,14 @@ attn_prefill_kernel(const PfArgs a, const __grid_constant__ CUtensorMap tm_q, co
           // lazy rescale: m only moves when a tile exceeds it by more than 2^kTau, so P <= 2^kTau and the accumulator in
           // TMEM is rarely touched.  P V of the tile before has retired: s_full was committed after it.
           constexpr float kTau = 7.0f;
-          const bool up = top > m + kTau;
+          // +inf turns m, and with it the row's sum and accumulator, into NaN.
+          const bool up = !(top <= m + kTau);
           if (__any_sync(0xffffffffu, up)) {               // the same in both warps of the pair
-            const float m_new = up ? top : m;
-            const float alpha = ex2(m - m_new);
+            const float m_new = up ? top + (top - top) : m;
+            float s0, s1, s2, s3;
+            unpack2(l0, s0, s1);
+            unpack2(l1, s2, s3);
+            const float alpha = fmaxf(fmaxf(s0, s1), fmaxf(s2, s3)) < kNanSum ? ex2(m - m_new) : NAN;
             const f32x2 al = pack2(alpha, alpha);
             l0 = fma2(l0, al, 0ull);
             l1 = fma2(l1, al, 0ull);
@@ -517,7 +525,7 @@ attn_prefill_kernel(const PfArgs a, const __grid_constant__ CUtensorMap tm_q, co
         unpack2(l1, s2, s3);
         const float l_own = (s0 + s1) + (s2 + s3), l_other = exchange(l_own);
         const float l = l_own + l_other;
-        const float fin = l > 0.f ? 1.0f / l : 0.f;
+        const float fin = l > 0.f ? (l < kNanSum ? 1.0f / l : NAN) : 0.f;      // a NaN sum: the accumulator holds them too
         const bool row_ok = li < n_valid;
         uint4* dst = reinterpret_cast<uint4*>(a.out + (static_cast<size_t>(r0 + li / a.group) * a.nq + w.kvh * a.group + li % a.group) * 128 + half * 64);
 #pragma unroll 1

@@ -83,6 +83,49 @@ def test_prefill_attention_negative_scale():
     assert torch.equal(a, b)
 
 
+def _nonfinite_case():
+    rows, nq, nkv, hd, dev = 300, 8, 2, 128, "cuda"
+    g = torch.Generator(device=dev).manual_seed(5)
+    kc = torch.randn(6, 64, nkv, hd, device=dev, generator=g).bfloat16()
+    vc = torch.randn(6, 64, nkv, hd, device=dev, generator=g).bfloat16()
+    pt = torch.tensor([[3, 1, 5, 2, 4]], dtype=torch.int32, device=dev)
+    seq = torch.zeros(rows, dtype=torch.int32, device=dev)
+    pos = torch.arange(rows, dtype=torch.int32, device=dev)
+    q = torch.randn(rows, nq, hd, device=dev, generator=g).bfloat16()
+    return q, kc, vc, pt, seq, pos
+
+
+# the exponentials of a tile take two ways, chosen by the key's place in its group of sixteen
+@pytest.mark.parametrize("t", list(range(32, 48)) + [0, 63, 64, 127, 129, 299])
+@pytest.mark.parametrize("value", ["nan", "inf"])
+def test_prefill_nonfinite_scores_reach_the_rows_that_see_them(t, value):
+    """A NaN or infinite score makes NaN of every row that attends to its key and of no other."""
+    from plow_b200.ops import gqa
+    q, kc, vc, pt, seq, pos = _nonfinite_case()
+    kc[pt[0, t // 64].long(), t % 64, :, 0] = float(value)
+    q[:, :, 0] = q[:, :, 0].abs() + 0.5                       # the infinite product is positive
+    ws = gqa.AttnWorkspace(len(pos), 8, 2, 128, 320, "cuda", max_splits=1)
+    out = gqa.attention(q, kc, vc, pt, seq, pos, ws)
+    assert out[t:].isnan().all()
+    assert out[:t].isfinite().all()
+
+
+def test_prefill_hidden_cells_weigh_nothing():
+    """Cells behind the rows' end and before their windows hold the largest finite values."""
+    from plow_b200.ops import gqa
+    q, kc, vc, pt, seq, pos = _nonfinite_case()
+    rows, window = len(pos), 40
+    pos = pos + 15
+    want = _ref(q, kc, vc, pt, seq, pos, window)
+    flat = vc[pt[0].long()].view(320, 2, 128)
+    t = torch.arange(320, device="cuda")
+    flat[(t > int(pos[-1])) | (t <= int(pos[0]) - window)] = 3.3e38
+    vc[pt[0].long()] = flat.view(5, 64, 2, 128)
+    ws = gqa.AttnWorkspace(rows, 8, 2, 128, 320, "cuda", max_splits=1)
+    out = gqa.attention(q, kc, vc, pt, seq, pos, ws, window=window)
+    assert (out.float() - want).norm() / want.norm() < 5e-3
+
+
 @pytest.mark.parametrize("rows,nq,nkv,pair_mode,norm,kv8,pad", [
     (3, 32, 8, 0, False, False, 0), (70, 32, 8, 1, True, False, 4), (300, 8, 1, 0, True, True, 0), (5, 4, 4, 1, False, True, 0),
     (9, 16, 2, 0, False, False, 2)])
