@@ -76,6 +76,10 @@ template <bool KV8> struct DecCfg {
   // stage only, and a parity wait cannot tell a phase from the one two before it.
   static constexpr int kStages = KV8 ? 8 : 4;
   static_assert(kStages % 4 == 0, "a stage belongs to one group of warps");
+  // Pages whose scales are on their way.  The producer asks for a page once the one kStages before it is consumed, which it has then
+  // long announced.
+  static constexpr uint32_t kScaleLag = 3;
+  static_assert(kScaleLag + 4 < kStages || !KV8, "every group of warps has a page that is announced");
   static constexpr int kTile = KV8 ? 8192 : 16384;               // one page of keys or values of a head
   static constexpr int kStage = 2 * kTile + (KV8 ? 512 : 0);     // + 64 key and 64 value scales
   // ring, control, then two merge areas: [8 warps][heads][132] f32
@@ -133,7 +137,7 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
   const int G = uncut ? a.rows * a.nkv : min(static_cast<int>(gridDim.x), (T + 3) / 4);
   if (static_cast<int>(blockIdx.x) >= G) return;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kS; ++s) { mbar_init(&full[s], KV8 ? 33 : 1); mbar_init(&empty[s], 2); }
+    for (int s = 0; s < kS; ++s) { mbar_init(&full[s], KV8 ? 2 : 1); mbar_init(&empty[s], 2); }
     for (int i = 0; i < 2; ++i) { mbar_init(&area_full[i], 8); mbar_init(&area_free[i], 3); }
     *abort_flag = 0;
     fence_mbar_init();
@@ -194,7 +198,8 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
             }
           }
           if constexpr (KV8) {
-            // scales of the 64 tokens: key scales, then value scales
+            // scales of the 64 tokens: key scales, then value scales.  Lane 0 arrives for them once every lane has seen its own copies
+            // of a page complete, kScaleLag pages later
             const float* src = a.kv_scale + static_cast<size_t>(page) * 64 * 2 * a.nkv + c.kvh;
             const uint32_t dst = smem_u32(st + 2 * Cfg::kTile);
 #pragma unroll
@@ -203,13 +208,23 @@ __device__ void gqa_decode_body(const DecArgs& a, const CUtensorMap* tm_k, const
               const float* g = src + static_cast<size_t>(e & 63) * 2 * a.nkv + (e >= 64 ? a.nkv : 0);
               asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst + e * 4), "l"(g) : "memory");
             }
-            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(&full[s])) : "memory");
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            if (k >= Cfg::kScaleLag) {
+              asm volatile("cp.async.wait_group %0;" ::"n"(Cfg::kScaleLag) : "memory");
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&full[(k - Cfg::kScaleLag) % kS]);
+            }
           }
         }
       }
       p += c.n;
     }
-    if (KV8) asm volatile("cp.async.wait_all;" ::: "memory");
+    if constexpr (KV8) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncwarp();
+      if (ok && lane == 0)
+        for (uint32_t j = k > Cfg::kScaleLag ? k - Cfg::kScaleLag : 0; j < k; ++j) mbar_arrive(&full[j % kS]);
+    }
   } else if (warp < 8) {
     // ------------------------------------------------------------------ consumers
     const int group = warp >> 1, tok0 = (warp & 1) * 32;     // which of four pages in turn, which 32 of its tokens

@@ -124,3 +124,19 @@ def test_zero_value_scales(zero, form):
     torch.cuda.synchronize()
     native.check_status()
     assert (out - ref).norm() <= 6e-3 * ref.norm()            # "all": exactly zero
+
+
+@pytest.mark.parametrize("kv8", [False, True])
+def test_repeats_bit_for_bit(kv8):
+    """Every SM at work on many pages: the ring, the scales and the fold give the same bits each time."""
+    from plow_b200.ops import gqa, native
+    lens = torch.randint(512, 4353, (64,), generator=torch.Generator().manual_seed(4)).tolist()
+    q, kc, vc, pt, seq, pos, ks, _, _ = _case(lens, 32, 8, kv8, 21)
+    ws = gqa.AttnWorkspace(64, 32, 8, 128, 4352, "cuda")
+    first = gqa.attention(q, kc, vc, pt, seq, pos, ws, kv_scale=ks)
+    bad = torch.zeros((), dtype=torch.int64, device="cuda")
+    for _ in range(300):
+        bad += (gqa.attention(q, kc, vc, pt, seq, pos, ws, kv_scale=ks) != first).any()
+    torch.cuda.synchronize()
+    native.check_status()
+    assert int(bad) == 0
