@@ -56,6 +56,10 @@ __device__ __forceinline__ float hash_uniform(unsigned long long seed, unsigned 
   return static_cast<float>(z >> 40) * (1.0f / 16777216.0f);   // [0, 1)
 }
 
+// largest of three, NaN if any is one: one such logit leaves the row without probabilities
+__device__ __forceinline__ float max_nan(float a, float b, float c) { float r; asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c)); return r; }
+__device__ __forceinline__ float max_nan(float a, float b) { return max_nan(a, b, b); }
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -470,24 +474,29 @@ sample_kernel(int* out, const float* logits, int ld, int V, int slice, int in_sm
       float4 v = reinterpret_cast<const float4*>(lg)[i];
       v.x *= invT; v.y *= invT; v.z *= invT; v.w *= invT;
       reinterpret_cast<float4*>(r.xs)[i] = v;
-      mx = fmaxf(mx, fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
+      mx = max_nan(max_nan(mx, v.x, v.y), v.z, v.w);
     }
 #pragma unroll 8
     for (int i = 4 * nq + r.tid; i < r.n; i += kThreads) {
       const float v = lg[i] * invT;
       if (r.in_smem) r.xs[i] = v;
-      mx = fmaxf(mx, v);
+      mx = max_nan(mx, v);
     }
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  for (int o = 16; o > 0; o >>= 1) mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   if (r.lane == 0) sh.part[r.ex][r.warp].f = mx;
   {
     const int buf = r.exchange();
     mx = -INFINITY;
-    for (int q = 0; q < r.nc; ++q) mx = fmaxf(mx, r.lane < kWarps ? r.peer(q)->part[buf][r.lane].f : -INFINITY);
+    for (int q = 0; q < r.nc; ++q) mx = max_nan(mx, r.lane < kWarps ? r.peer(q)->part[buf][r.lane].f : -INFINITY);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    for (int o = 16; o > 0; o >>= 1) mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  }
+  if (mx != mx) {
+    if (r.rank == 0 && r.tid == 0) out[row] = -1;
+    r.cl().sync();      // other CTAs may still read this one's maximum
+    return;
   }
   const float u = u_in ? u_in[row] : hash_uniform(seed ? seed[row] : 0ull, step);
   const float tp = top_p ? top_p[row] : 1.0f;

@@ -62,6 +62,23 @@ def test_sampler_sizes(V, ld):
         _check(logits, temperature, top_k, top_p, min_p, u, got)
 
 
+@pytest.mark.parametrize("V", [3, 700, 9000, 60000, 361000])
+def test_sampler_nonfinite_rows(V):
+    """A NaN or +inf among the scaled logits leaves no probabilities: no token, whatever the filters.  Greedy rows order by value."""
+    from plow_b200.ops import sampler
+    g = torch.Generator(device="cuda").manual_seed(V)
+    rows = torch.randn(7, V, device="cuda", generator=g)
+    for r, (at, v) in enumerate([(0, "nan"), (V // 2, "nan"), (V - 1, "-nan"), (V - 1, "inf"), (1, "-inf"), (0, "nan"), (2, "inf")]):
+        rows[r, at] = float(v)
+    temp = torch.tensor([1.0, 0.7, 1.0, 1.0, 1.0, 0.0, 0.0], device="cuda")
+    for k, p, m in ((0, 1.0, 0.0), (1, 1.0, 0.0), (50, 0.9, 0.1), (3000, 1.0, 0.0), (0, 0.5, 0.0)):
+        kk = torch.full((7,), k, dtype=torch.int32, device="cuda")
+        got = sampler.sample(rows, temp, kk, torch.full_like(temp, p), torch.full_like(temp, m), u=torch.full_like(temp, 0.4)).tolist()
+        assert got[:4] == [-1] * 4, (k, p)
+        assert 0 <= got[4] < V and got[4] != 1
+        assert got[5] == 0 and got[6] == 2
+
+
 @pytest.mark.parametrize("V", [500, 9000, 60000])
 def test_sampler_ties_and_degenerate_rows(V):
     """All logits equal, two values, one live token, masked rows: every element at a cut value is kept."""
