@@ -35,7 +35,10 @@ def _ref(q, kc, vc, pt, seq, pos, window):
 @pytest.mark.parametrize("runs,idle,nq,nkv,window", [
     ([(257, 0)], 0, 32, 8, 0), ([(300, 0), (1, 700), (65, 63)], 0, 32, 8, 0), ([(129, 1), (127, 64), (64, 128)], 3, 8, 8, 0),
     ([(1, 0), (2, 62), (31, 96), (33, 5), (256, 191)], 1, 16, 2, 0), ([(500, 77)], 0, 8, 1, 100), ([(330, 1000)], 0, 32, 8, 64),
-    ([(1, 40 + 13 * i) for i in range(260)], 0, 32, 8, 0), ([(400, 3)], 0, 4, 4, 129)])
+    ([(1, 40 + 13 * i) for i in range(260)], 0, 32, 8, 0), ([(400, 3)], 0, 4, 4, 129),
+    # more one-tile items than SMs: chunks of two tiles, cut from each run's own first row
+    ([(650, 77)], 0, 32, 8, 100), ([(1300, 0)], 0, 16, 2, 0), ([(2500, 30), (31, 0)], 2, 8, 8, 0), ([(33, 100 + i) for i in range(21)], 1, 32, 8, 0),
+    ([(15, 3 * i) for i in range(70)], 0, 32, 8, 0), ([(64, 0), (65, 10), (63, 90), (128, 1), (129, 0), (1, 700), (2, 5), (190, 40)], 1, 32, 8, 0)])
 def test_prefill_attention(runs, idle, nq, nkv, window):
     from plow_b200.ops import gqa, native
     hd, dev = 128, "cuda"
@@ -65,6 +68,27 @@ def test_prefill_attention(runs, idle, nq, nkv, window):
     assert rel < 5e-3, rel
     assert (out[live].float() - want[live]).abs().max() < 4e-2
     assert (out[~live] == 7.0).all()
+
+
+def test_prefill_attention_default_workspace():
+    """The workspace's own split count at the served head ratio: whole and partly filled second tiles, more items than SMs."""
+    from plow_b200.ops import gqa, native
+    runs, nq, nkv, hd, dev = [(700, 0), (1, 900), (33, 64), (520, 300), (20, 5), (2, 1000), (150, 0)], 32, 8, 128, "cuda"
+    g = torch.Generator(device=dev).manual_seed(9)
+    per = max((n + p + 63) // 64 for n, p in runs)
+    kc = torch.randn(len(runs) * per, 64, nkv, hd, device=dev, generator=g).bfloat16()
+    vc = torch.randn(len(runs) * per, 64, nkv, hd, device=dev, generator=g).bfloat16()
+    pt = torch.randperm(len(runs) * per, device=dev, generator=g).int().view(len(runs), per).contiguous()
+    seq = torch.cat([torch.full((n,), i, dtype=torch.int32) for i, (n, _) in enumerate(runs)]).to(dev)
+    pos = torch.cat([torch.arange(p, p + n, dtype=torch.int32) for n, p in runs]).to(dev)
+    q = torch.randn(len(pos), nq, hd, device=dev, generator=g).bfloat16()
+    ws = gqa.AttnWorkspace(len(pos), nq, nkv, hd, per * 64, dev)
+    assert ws.max_splits == 1                 # this many rows fill the chip unsplit: the two-tile kernel
+    out = gqa.attention(q, kc, vc, pt, seq, pos, ws)
+    torch.cuda.synchronize()
+    native.check_status()
+    want = _ref(q, kc, vc, pt, seq, pos, 0)
+    assert (out.float() - want).norm() / want.norm() < 5e-3
 
 
 def test_prefill_attention_negative_scale():
