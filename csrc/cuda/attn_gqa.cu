@@ -42,7 +42,8 @@
 namespace plow {
 
 constexpr int kGqaPage = 64;
-constexpr int kGqaThreads = 192;   // TMA warp, MMA warp, 4 softmax warps (and 4 converter warps for the e4m3 cache)
+constexpr int kGqaThreads = 192;   // TMA warp, MMA warp, 4 softmax warps
+constexpr int kGqaThreads8 = 320;  // + 4 converter warps (e4m3 cache)
 constexpr int kGqaRaw = 3;         // raw e4m3 tiles in flight; 4 operand stages behind them
 
 // Rows from which an unsplit bf16 call takes the two-tile kernel of attn_prefill.cu: its items are up to twice as long, so
@@ -69,7 +70,8 @@ struct GqaArgs {
 };
 
 // HDQ = width of a query / key row, HDV = width of a value row.
-template <int HDQ, int HDV, bool KV8 = false> struct GqaCfg {
+// DEC: the kernel also holds the decode body of attn_decode.cuh.
+template <int HDQ, int HDV, bool KV8 = false, bool DEC = false> struct GqaCfg {
   static constexpr int kSlabsQ = HDQ / 64;               // 64-column (128-byte) slabs per query / key row
   static constexpr int kSlabsV = HDV / 64;
   static constexpr int kQBytes = kSlabsQ * 128 * 128;
@@ -84,7 +86,9 @@ template <int HDQ, int HDV, bool KV8 = false> struct GqaCfg {
   // per operand stage: 64 S-column and 64 P-column factors; then a ring of 128 page numbers for the converter warps
   static constexpr int kColBytes = KV8 ? kStages * 128 * 4 + 128 * 4 : 0;
   static constexpr int kSmem = 1024 + kQBytes + kStages * kStageBytes + kRawBytes + kColBytes + 1024;
-  static constexpr int kThreads = HDQ == 128 ? kDecThreads : kGqaThreads;     // as many as the decode body has
+  // With the decode body the block has that one's threads, and 168 registers a thread instead of 204 and 255: calls that cannot be
+  // decode steps take the kernel without it (512 rows over the e4m3 cache 58.4 us, with the body 60.7).
+  static constexpr int kThreads = DEC ? kDecThreads : (KV8 ? kGqaThreads8 : kGqaThreads);
   static constexpr int kTmemCols = HDV <= 128 ? 256 : 512; // S: 2 x 64, O: HDV
   static_assert(kStages >= 2, "K/V stages do not fit");
   static_assert(kSmem <= 227 * 1024, "shared memory budget");
@@ -175,21 +179,21 @@ gqa_plan_small(const int* seq, const int* pos, int rows, int tq, int nkv, int wi
   if (r == 0) { *n_items = min(n_sh, cap); sc.plan[0] = 0; }
 }
 
-template <int HDQ, int HDV, bool KV8 = false>
-__global__ void __launch_bounds__((GqaCfg<HDQ, HDV, KV8>::kThreads), 1)
+template <int HDQ, int HDV, bool KV8, bool DEC>
+__global__ void __launch_bounds__((GqaCfg<HDQ, HDV, KV8, DEC>::kThreads), 1)
 gqa_attn_kernel(const GqaArgs a, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v) {
   plow::pdl_launch_dependents();
   plow::pdl_wait();
-  if constexpr (HDQ == 128) {
+  if constexpr (DEC) {
     // a decode step: the streaming form (the plan kernel decided)
-    if (a.dec && *static_cast<const int*>(a.dec) == 1) {
+    if (*static_cast<const int*>(a.dec) == 1) {
       const DecArgs d = {a.dec, a.q, a.page_table, a.pos, a.seq, a.kv_scale, a.out, a.status, a.rows, a.nq, a.nkv, a.group, a.max_pages, a.window, a.scale_log2e};
       gqa_decode_body<KV8>(d, &tm_k, &tm_v);
       return;
     }
   }
-  using Cfg = GqaCfg<HDQ, HDV, KV8>;
+  using Cfg = GqaCfg<HDQ, HDV, KV8, DEC>;
   constexpr int HD = HDV;      // width of the accumulator rows
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -819,39 +823,23 @@ rope_kv128_kernel(__nv_bfloat16* q_out, const __nv_bfloat16* qkv, int ld_qkv, __
   }
 }
 
-template <int HD>
+// kc / vc: bf16 [tokens][nkv][HD], or e4m3 bytes (KV8).
+template <int HD, bool KV8, bool DEC>
 int launch_gqa(const GqaArgs& a, const void* q, const void* kc, const void* vc, int64_t n_pages, int grid, cudaStream_t stream) {
-  using Cfg = GqaCfg<HD, HD>;
-  constexpr int kSmem = HD == 128 ? (Cfg::kSmem > DecCfg<false>::smem(kDecMaxGroup) ? Cfg::kSmem : DecCfg<false>::smem(kDecMaxGroup)) : Cfg::kSmem;
+  using Cfg = GqaCfg<HD, HD, KV8, DEC>;
+  constexpr int kSmem = DEC && DecCfg<KV8>::smem(kDecMaxGroup) > Cfg::kSmem ? DecCfg<KV8>::smem(kDecMaxGroup) : Cfg::kSmem;
   static_assert(kSmem <= 227 * 1024, "shared memory budget");
+  constexpr int kCell = KV8 ? 1 : 2;
   CUtensorMap tq, tk, tv;
   int r = make_tmap_3d(&tq, q, 2, HD, a.nq, a.rows, HD * 2, static_cast<uint64_t>(a.nq) * HD * 2, a.group, 128 / a.group, 128);
   if (r) return 1100 + r;
-  r = make_tmap_3d(&tk, kc, 2, HD, a.nkv, static_cast<uint64_t>(n_pages) * kGqaPage, HD * 2, static_cast<uint64_t>(a.nkv) * HD * 2, 1, kGqaPage, 128);
+  r = make_tmap_3d(&tk, kc, kCell, HD, a.nkv, static_cast<uint64_t>(n_pages) * kGqaPage, HD * kCell, static_cast<uint64_t>(a.nkv) * HD * kCell, 1, kGqaPage, 128);
   if (r) return 1200 + r;
-  r = make_tmap_3d(&tv, vc, 2, HD, a.nkv, static_cast<uint64_t>(n_pages) * kGqaPage, HD * 2, static_cast<uint64_t>(a.nkv) * HD * 2, 1, kGqaPage, 128);
+  r = make_tmap_3d(&tv, vc, kCell, HD, a.nkv, static_cast<uint64_t>(n_pages) * kGqaPage, HD * kCell, static_cast<uint64_t>(a.nkv) * HD * kCell, 1, kGqaPage, 128);
   if (r) return 1300 + r;
   static DeviceOnce attr;
-  if (ensure_smem(attr, gqa_attn_kernel<HD, HD>, kSmem) != cudaSuccess) return 3000;
-  plow::launch_serial(gqa_attn_kernel<HD, HD>, dim3(grid), dim3(Cfg::kThreads), kSmem, stream, a, tq, tk, tv);
-  return 0;
-}
-
-// e4m3 cache: kc / vc are bytes [n_pages*64][nkv][HD]; raw tiles of 128 bytes x 64 tokens per load.
-template <int HD>
-int launch_gqa8(const GqaArgs& a, const void* q, const void* kc, const void* vc, int64_t n_pages, int grid, cudaStream_t stream) {
-  using Cfg = GqaCfg<HD, HD, true>;
-  static_assert(DecCfg<true>::smem(kDecMaxGroup) <= Cfg::kSmem, "the decode body fits the tile kernel's shared memory");
-  CUtensorMap tq, tk, tv;
-  int r = make_tmap_3d(&tq, q, 2, HD, a.nq, a.rows, HD * 2, static_cast<uint64_t>(a.nq) * HD * 2, a.group, 128 / a.group, 128);
-  if (r) return 1100 + r;
-  r = make_tmap_3d(&tk, kc, 1, HD, a.nkv, static_cast<uint64_t>(n_pages) * kGqaPage, HD, static_cast<uint64_t>(a.nkv) * HD, 1, kGqaPage, 128);
-  if (r) return 1200 + r;
-  r = make_tmap_3d(&tv, vc, 1, HD, a.nkv, static_cast<uint64_t>(n_pages) * kGqaPage, HD, static_cast<uint64_t>(a.nkv) * HD, 1, kGqaPage, 128);
-  if (r) return 1300 + r;
-  static DeviceOnce attr;
-  if (ensure_smem(attr, gqa_attn_kernel<HD, HD, true>, Cfg::kSmem) != cudaSuccess) return 3000;
-  plow::launch_serial(gqa_attn_kernel<HD, HD, true>, dim3(grid), dim3(Cfg::kThreads), Cfg::kSmem, stream, a, tq, tk, tv);
+  if (ensure_smem(attr, gqa_attn_kernel<HD, HD, KV8, DEC>, kSmem) != cudaSuccess) return 3000;
+  plow::launch_serial(gqa_attn_kernel<HD, HD, KV8, DEC>, dim3(grid), dim3(Cfg::kThreads), kSmem, stream, a, tq, tk, tv);
   return 0;
 }
 
@@ -910,8 +898,10 @@ int plow_gqa_attention(const void* q, const void* kc, const void* vc, int64_t n_
   a.scale_log2e = softmax_scale * 1.4426950408889634f;
   a.kv_scale = kv_scale;
   if (!dec && item_cap < grid) grid = item_cap;
-  int r = kv_scale ? launch_gqa8<128>(a, q, kc, vc, n_pages, grid, stream)
-          : hd == 128 ? launch_gqa<128>(a, q, kc, vc, n_pages, grid, stream) : launch_gqa<256>(a, q, kc, vc, n_pages, grid, stream);
+  int r;
+  if (hd == 256) r = launch_gqa<256, false, false>(a, q, kc, vc, n_pages, grid, stream);
+  else if (kv_scale) r = dec ? launch_gqa<128, true, true>(a, q, kc, vc, n_pages, grid, stream) : launch_gqa<128, true, false>(a, q, kc, vc, n_pages, grid, stream);
+  else r = dec ? launch_gqa<128, false, true>(a, q, kc, vc, n_pages, grid, stream) : launch_gqa<128, false, false>(a, q, kc, vc, n_pages, grid, stream);
   if (r) return r;
   if (max_splits > 1)
     plow::launch_serial(gqa_merge_kernel, dim3(rows, nq), dim3(128), 0, stream, opart, lse, row_ns, nq, max_splits, hd, static_cast<__nv_bfloat16*>(out));
