@@ -23,6 +23,7 @@
 #include <stdint.h>
 
 #include "launch.cuh"
+#include "tmap.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -100,7 +101,8 @@ struct Row {
   __device__ float x(int i) const { return in_smem ? xs[i] : lg[i] * invT; }
   __device__ Shared* peer(int r) { return cl().map_shared_rank(sh, r); }
   // this CTA's part values are in part[ex]; afterwards every CTA may read all of them
-  __device__ int exchange() { cl().sync(); const int b = ex; ex ^= 1; return b; }
+  __device__ int exchange() { sync(); const int b = ex; ex ^= 1; return b; }
+  __device__ void sync() const { if (nc > 1) cl().sync(); else __syncthreads(); }
 
   // f(x) for every element of the slice, four at a time from shared memory
   template <class F>
@@ -402,7 +404,7 @@ __device__ void finish_in_list(Row& r, int n, const uint32_t* sk, float x_thr, f
 }
 
 __global__ void __launch_bounds__(kThreads)
-sample_kernel(int* out, const float* logits, int ld, int V, int slice, int in_smem, const float* temperature, const int* top_k,
+sample_kernel(int* out, const float* logits, int ld, int V, int slice, int in_smem, int greedy_alone, const float* temperature, const int* top_k,
               const float* top_p, const float* min_p, const float* u_in, const unsigned long long* seed,
               unsigned long long step) {
   plow::pdl_launch_dependents();
@@ -429,18 +431,34 @@ sample_kernel(int* out, const float* logits, int ld, int V, int slice, int in_sm
   const bool quads = (reinterpret_cast<uintptr_t>(lg) & 15) == 0;      // the row's start decides: ld need not be a multiple of 4
   const float T = temperature ? temperature[row] : 1.0f;
   if (T <= 0.f) {
+    if (greedy_alone) {
+      // The CTAs do not fit the chip at once: a greedy row, which reads its logits once, gives its cluster's places back (128 rows x
+      // 128256, all greedy: 36 us, 44 with the whole cluster at work; with all resident one row of 128256 takes 13 us, alone 25).
+      if (r.rank) return;
+      r.n = V; r.nc = 1;
+    }
     // arg-max, lowest index on ties: a thread sees its indices in ascending order, then packed (ordered value, ~index)
     uint32_t bk = 0, bi = 0;
     bool any = false;
     auto see = [&](float v, int i) { const uint32_t kx = ordered_key(v); if (!any || kx > bk) { bk = kx; bi = i; any = true; } };
     const int nq = quads ? r.n / 4 : 0;
-#pragma unroll 8
-    for (int i = r.tid; i < nq; i += kThreads) {
+    int i = r.tid;
+    for (; i + 7 * kThreads < nq; i += 8 * kThreads) {
+      float4 v[8];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) v[t] = reinterpret_cast<const float4*>(lg)[i + t * kThreads];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        const int at = 4 * (i + t * kThreads);
+        see(v[t].x, at); see(v[t].y, at + 1); see(v[t].z, at + 2); see(v[t].w, at + 3);
+      }
+    }
+    for (; i < nq; i += kThreads) {
       const float4 v = reinterpret_cast<const float4*>(lg)[i];
       see(v.x, 4 * i); see(v.y, 4 * i + 1); see(v.z, 4 * i + 2); see(v.w, 4 * i + 3);
     }
 #pragma unroll 8
-    for (int i = 4 * nq + r.tid; i < r.n; i += kThreads) see(lg[i], i);
+    for (i = 4 * nq + r.tid; i < r.n; i += kThreads) see(lg[i], i);
     unsigned long long best = any ? (static_cast<unsigned long long>(bk) << 32) | (0xFFFFFFFFu - (r.base + bi)) : 0ull;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -454,7 +472,7 @@ sample_kernel(int* out, const float* logits, int ld, int V, int slice, int in_sm
       for (int w = 1; w < kWarps; ++w) best = bw[w] > best ? bw[w] : best;
       bw[0] = best;
     }
-    r.cl().sync();
+    r.sync();
     if (r.rank == 0 && r.tid == 0) {
       for (int q = 1; q < r.nc; ++q) {
         const unsigned long long t = *r.cl().map_shared_rank(bw, q);
@@ -462,7 +480,7 @@ sample_kernel(int* out, const float* logits, int ld, int V, int slice, int in_sm
       }
       out[row] = static_cast<int>(0xFFFFFFFFu - static_cast<uint32_t>(best & 0xFFFFFFFFu));
     }
-    r.cl().sync();        // the other CTAs' words stay readable until here
+    r.sync();        // the other CTAs' words stay readable until here
     return;
   }
   const float invT = r.invT = 1.0f / fmaxf(T, 1e-6f);
@@ -495,7 +513,7 @@ sample_kernel(int* out, const float* logits, int ld, int V, int slice, int in_sm
   }
   if (mx != mx) {
     if (r.rank == 0 && r.tid == 0) out[row] = -1;
-    r.cl().sync();      // other CTAs may still read this one's maximum
+    r.sync();      // other CTAs may still read this one's maximum
     return;
   }
   const float u = u_in ? u_in[row] : hash_uniform(seed ? seed[row] : 0ull, step);
@@ -515,7 +533,7 @@ sample_kernel(int* out, const float* logits, int ld, int V, int slice, int in_sm
     if (k <= kCap && above + own <= kCap) {
       // every candidate fits the list: the first CTA finishes the row there
       const int n = gather(r, [&](float x) { return iv.reached(x); });
-      r.cl().sync();
+      r.sync();
       if (r.rank == 0) {
         const uint32_t* sk = sorted_list(r, min(n, kCap));
         finish_in_list(r, min(n, kCap), sk, key_value(sk[min(k, n) - 1]), mx, 0.f, nucleus, tp, mp, u, out + row);
@@ -526,15 +544,15 @@ sample_kernel(int* out, const float* logits, int ld, int V, int slice, int in_sm
       x_thr = key_value(iv.klo);
     } else {
       const int n = min(kCap, gather(r, [&](float x) { return iv.inside(x); }));
-      r.cl().sync();
+      r.sync();
       if (r.rank == 0) {
         const int at = min(n - 1, max(0, k - static_cast<int>(above) - 1));
         const uint32_t* sk = sorted_list(r, n);
         if (r.tid == 0) sh.bc_f = n > 0 ? key_value(sk[at]) : -INFINITY;
       }
-      r.cl().sync();
+      r.sync();
       x_thr = r.peer(0)->bc_f;
-      r.cl().sync();
+      r.sync();
     }
   }
   // exponentials stand for the probabilities throughout: a cut on p = e / Z is a cut on e, the draw compares with u times
@@ -554,7 +572,7 @@ sample_kernel(int* out, const float* logits, int ld, int V, int slice, int in_sm
         n = gather(r, [&](float x) { return iv.reached(x); });
         if (n <= kCap) {
           // a peaked row: everything that can be kept fits the list
-          r.cl().sync();
+          r.sync();
           if (r.rank == 0) finish_in_list(r, n, sorted_list(r, n), x_thr, mx, c.all, true, tp, mp, u, out + row);
           return;
         }
@@ -573,15 +591,15 @@ sample_kernel(int* out, const float* logits, int ld, int V, int slice, int in_sm
       if (iv.single()) {
         cut = e_of(key_value(iv.klo));
       } else {
-        r.cl().sync();
+        r.sync();
         if (r.rank == 0) {
           const uint32_t* sk = sorted_list(r, n);
           const int pos = n > 0 ? first_reaching(r, sk, n, above, target, e_of) : 0;
           if (r.tid == 0) sh.bc_f = n > 0 ? e_of(key_value(sk[pos])) : 0.f;
         }
-        r.cl().sync();
+        r.sync();
         cut = r.peer(0)->bc_f;
-        r.cl().sync();
+        r.sync();
       }
       e_cut = fmaxf(e_cut, cut);
     }
@@ -669,7 +687,7 @@ sample_kernel(int* out, const float* logits, int ld, int V, int slice, int in_sm
     if (pick < 0) pick = kept;     // rounding left the target at or past the part's end: its last kept index
     if (r.lane == 0) out[row] = pick >= 0 ? r.base + pick : -1;
   }
-  r.cl().sync();                     // other CTAs may still read this one's sums
+  r.sync();                     // other CTAs may still read this one's sums
 }
 
 }  // namespace
@@ -681,11 +699,13 @@ extern "C" {
 int plow_sample(int* out, const float* logits, int ld, int rows, int V, const float* temperature, const int* top_k,
                 const float* top_p, const float* min_p, const float* u, const void* seed, uint64_t step, void* stream) {
   if (rows <= 0 || V <= 0) return -1;
-  // CTAs per row: as many as it takes for the slices to fit two CTAs to an SM, and while the rows alone leave SMs idle
-  // up to eight (a slice is not cut below 1024 elements); both ends measured, see above.
+  const int room = 2 * plow::sm_count();
+  // CTAs per row: as many as it takes for the slices to fit two CTAs to an SM, and beyond that up to eight while all CTAs are resident
+  // at once (64 rows x 8192, no filter: 15.7 us as 256 CTAs, 28.1 as 512) and a slice has 2048 elements (32 rows x 8192, no filter:
+  // 14.3 us as slices of 2048, 17.6 of 1024).
   int nc = 1;
   while (nc < kMaxCluster && (V + nc - 1) / nc > kSlice) nc <<= 1;
-  while (nc < kMaxCluster && static_cast<long long>(rows) * nc < 2 * 148 && V / (2 * nc) >= 1024) nc <<= 1;
+  while (nc < kMaxCluster && static_cast<long long>(rows) * 2 * nc <= room && V / (2 * nc) >= 2048) nc <<= 1;
   const int slice = ((V + nc - 1) / nc + 3) & ~3;
   const int in_smem = slice <= kSliceMax;
   const size_t smem = sizeof(float) * (kBins * kThreads + (in_smem ? slice : 0));
@@ -701,7 +721,7 @@ int plow_sample(int* out, const float* logits, int ld, int rows, int V, const fl
   at[0].val.clusterDim.x = nc; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, sample_kernel, out, logits, ld, V, slice, in_smem, temperature, top_k, top_p, min_p, u,
+  cudaError_t e = cudaLaunchKernelEx(&cfg, sample_kernel, out, logits, ld, V, slice, in_smem, static_cast<int>(static_cast<long long>(rows) * nc > room), temperature, top_k, top_p, min_p, u,
                                      static_cast<const unsigned long long*>(seed), static_cast<unsigned long long>(step));
   if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 4000 + static_cast<int>(e);

@@ -62,6 +62,25 @@ def test_sampler_sizes(V, ld):
         _check(logits, temperature, top_k, top_p, min_p, u, got)
 
 
+# CTAs per row 8 to 1, all resident at once or not; greedy rows then are one CTA's
+@pytest.mark.parametrize("rows,V,ld", [(37, 16384, 16384), (64, 9001, 9003), (74, 8192, 8192), (200, 4095, 4096), (310, 20003, 20005), (40, 150001, 150001)])
+def test_sampler_many_rows(rows, V, ld):
+    from plow_b200.ops import sampler
+    g = torch.Generator(device="cuda").manual_seed(V)
+    logits = (torch.randn(rows, ld, device="cuda", generator=g) * 2)[:, :V]
+    logits[:, V // 3] = logits[:, V - 1]                     # ties: the lowest index
+    r = torch.arange(rows, device="cuda")
+    top = torch.arange(0, rows, 4, device="cuda")
+    logits[top, V - 1] = logits[top, V // 3] = 30.0
+    temperature = torch.where(r % 2 == 0, 0.0, 0.8)
+    top_k = torch.where(r % 3 == 0, 40, 0).int()
+    top_p = torch.where(r % 5 == 0, 0.9, 1.0)
+    u = torch.rand(rows, device="cuda", generator=g)
+    got = sampler.sample(logits, temperature, top_k, top_p, torch.zeros(rows, device="cuda"), u=u)
+    assert (got[top].long() == V // 3).all()
+    _check(logits, temperature, top_k, top_p, torch.zeros(rows), u, got)
+
+
 @pytest.mark.parametrize("V", [3, 700, 9000, 60000, 361000])
 def test_sampler_nonfinite_rows(V):
     """A NaN or +inf among the scaled logits leaves no probabilities: no token, whatever the filters.  Greedy rows order by value."""
