@@ -7,7 +7,7 @@
 // Reference semantics: runtime/common/dev_isa.h:516-534 and :1083-1115 (7-pass radix select over a
 // monotone packed key, live token-granular kv_len), runtime/nvidia/op_dsa.cuh.
 //
-// Scores: one CTA per (eight 128-token tiles, query row).  A tile's keys are the A operand (M = 128 tokens),
+// Scores: one CTA per (up to eight 128-token tiles, query row).  A tile's keys are the A operand (M = 128 tokens),
 // the row's 64 index heads the B operand (N = 64), K = 128 e4m3: D[token][head] lands with one token
 // per TMEM lane, so the weighted ReLU sum over heads is a private 64-column loop per thread and the
 // score leaves the kernel with one coalesced store.  One warp keeps a ring of four tiles and two accumulators busy,
@@ -136,20 +136,20 @@ __global__ void dsa_q_prep_kernel(uint8_t* q8, float* w_out, const __nv_bfloat16
   if (lane == 0) w_out[r * kIdxHeads + h] = w[static_cast<size_t>(r) * ld_w + h] * sc;
 }
 
-constexpr int kScoreTiles = 8;            // 128-token tiles per CTA
+constexpr int kScoreTiles = 8;            // 128-token tiles per CTA at most
 constexpr int kScoreStages = 4;
 constexpr int kScoreSmem = 1024 + 8192 + kScoreStages * 16384 + 1024;
 
 __global__ void __launch_bounds__(160)
-dsa_score_kernel(float* scores, int ld_scores, const float* w, const float* kscale, const int* pos, const int* seq,
+dsa_score_kernel(float* scores, int ld_scores, int cta_tiles, const float* w, const float* kscale, const int* pos, const int* seq,
                  const int* page_table, int max_pages, int* status, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_q) {
   plow::pdl_launch_dependents();
   plow::pdl_wait();
-  const int r = blockIdx.y, t0 = blockIdx.x * 128 * kScoreTiles;
+  const int r = blockIdx.y, t0 = blockIdx.x * 128 * cta_tiles;
   const int len = pos[r] + 1;
   if (t0 >= len) return;
-  const int n_tiles = min(kScoreTiles, (len - t0 + 127) / 128);
+  const int n_tiles = min(cta_tiles, (len - t0 + 127) / 128);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* q_smem = smem;                 // 64 heads x 128 B
@@ -497,8 +497,12 @@ int plow_dsa_select(int* sel, float* scores, int ld_scores, void* q8, float* wq,
   if (rc) return 1200 + rc;
   static DeviceOnce attr;
   if (ensure_smem(attr, dsa_score_kernel, kScoreSmem) != cudaSuccess) return 3000;
-  plow::launch_serial(dsa_score_kernel, dim3((max_len + 128 * kScoreTiles - 1) / (128 * kScoreTiles), rows), dim3(160), kScoreSmem, stream, scores, ld_scores,
-                      wq, cache_scale, pos, seq, page_table, max_pages, status, tk, tq);
+  // tiles per CTA: as few as still fit the chip at once (three CTAs per SM).  A CTA takes its tiles one after the other: 8 rows of 1500
+  // tokens took 19.5 us at eight tiles, 15.3 at one.
+  const int tiles = (max_len + 127) / 128;
+  int per = kScoreTiles;
+  while (per > 1 && static_cast<long long>(rows) * ((2 * tiles + per - 1) / per) <= 3 * sm_count()) per >>= 1;
+  plow::launch_serial(dsa_score_kernel, dim3((tiles + per - 1) / per, rows), dim3(160), kScoreSmem, stream, scores, ld_scores, per, wq, cache_scale, pos, seq, page_table, max_pages, status, tk, tq);
   // CTAs per row: while the rows alone leave SMs idle or a CTA would hold over a quarter of its room (two to four stay
   // resident per SM), but none with under 1024 elements, where the cluster's barriers cost more than the passes
   int nc = 1;

@@ -17,6 +17,7 @@ def _order(scores, top_k):
     ([1, 0, 63, 64, 65, 127, 128, 129], 64, "rand"),
     ([1023, 1024, 1025, 1152, 2047, 2048, 2049, 2176], 2048, "rand"),
     ([4097, 8191, 16384, 10241, 500], 2048, "rand"),
+    ([16384, 1, 1000, 8191, 2305, 512] * 2, 2048, "rand"),           # four tiles a CTA (above: two; below: eight)
     ([5000] * 150 + [7, 4999], 512, "rand"),
     ([9000] * 300, 100, "rand"),
     ([6000, 2049, 12345], 2048, "few"),
