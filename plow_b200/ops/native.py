@@ -193,13 +193,26 @@ def profile_summary() -> list:
         e[1] += a.elapsed_time(b)
     PROFILE.clear()
     return sorted(((k, c, t) for k, (c, t) in agg.items()), key=lambda x: -x[2])
-_KERNELS_PER_CALL = {"plow_gqa_attention": 2, "plow_dsa_select": 3, "plow_mla_prefill_attention": 2, "plow_gdn": 2}
+
+
+_KERNELS_PER_CALL = {"plow_dsa_select": 3, "plow_mla_prefill_attention": 2}
+
+
+def _kernels(name: str, args) -> int:
+    """Kernels that a launcher starts with these arguments."""
+    if name == "plow_gqa_attention":
+        return 3 if args[14] > 1 else 2               # work list, attention, merge of the splits
+    if name == "plow_gdn":
+        return 3 if args[12] > 64 else 2              # beyond a decode step's rows long runs have a kernel of their own
+    if name == "plow_mla_decode":
+        return 1 + int(args[19]) + (args[17] is not None)      # work list and merge only if asked for
+    return _KERNELS_PER_CALL.get(name, 1)
 
 
 def call(name: str, *args) -> None:
     """Invoke a kernel launcher of libplow_cuda.so on the current stream (appended as last arg)."""
     lib = cuda_lib()
-    LAUNCHES["n"] += _KERNELS_PER_CALL.get(name, 1)
+    LAUNCHES["n"] += _kernels(name, args)
     fn = getattr(lib, name)
     if fn.argtypes is None:
         fn.argtypes = [_CT[c] for c in _SIGS[name]]
