@@ -913,14 +913,12 @@ int plow_gqa_attention(const void* q, const void* kc, const void* vc, int64_t n_
 // already rotated); kvb bf16 [n_tokens][heads][256]; krope bf16 [n_tokens][64]; vpt int32 [n_slots][max_pages]: tile i
 // of slot s covers tokens [64 vpt[s][i], 64 vpt[s][i] + 64) of kvb / krope; seq / pos int32 [rows] (pos < 0: the row is
 // not attended here); out bf16 [rows][heads*128].  Scratch: items (8 ints each, capacity item_cap), n_items (1 int), row_ns
-// int32 [rows].  Keys are never split (a chunk has an item for every head): the split arguments and their scratch are unused.
+// int32 [rows].  Keys are never split: a chunk has an item for every head.
 int plow_mla_prefill_attention(const void* q, const void* kvb, const void* krope, int64_t n_tokens, const int* vpt, int max_pages,
-                               const int* seq, const int* pos, int rows, int heads, int tiles_per_split, int max_splits,
-                               void* items, int item_cap, int* n_items, int* row_ns, float* opart, float* lse, void* out,
+                               const int* seq, const int* pos, int rows, int heads, void* items, int item_cap, int* n_items, int* row_ns, void* out,
                                float softmax_scale, int* status, void* stream_) {
   using namespace plow;
-  if (rows <= 0 || heads <= 0 || max_splits <= 0 || tiles_per_split <= 0 || n_tokens <= 0) return -1;
-  (void)opart; (void)lse;
+  if (rows <= 0 || heads <= 0 || n_tokens <= 0) return -1;
   PrefillArgs p = {q, kvb, kvb, krope, vpt, seq, pos, items, item_cap, n_items, row_ns, out, status,
                    n_tokens, rows, heads, heads, max_pages, 0, softmax_scale};
   const int rc = launch_attn_prefill(p, reinterpret_cast<cudaStream_t>(stream_));

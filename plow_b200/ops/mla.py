@@ -117,15 +117,12 @@ class PrefillWorkspace:
         self.kvb = torch.empty(budget, heads * 256, dtype=BF16, device=device)
         self.vpt = torch.zeros(n_slots, max_pages, dtype=torch.int32, device=device)
         chunks = (max_rows + 127) // 128 + n_slots
-        # one (128-row chunk, head) item per CTA visit: with 128 heads even a single chunk fills the GPU, so the keys of
-        # a chunk are never split
-        self.tiles_per_split = 1 << 20
-        self.max_splits = 1
-        self.item_cap = chunks * heads * self.max_splits
+        # chunks of up to two 128-row tiles, eight words each; the room also holds one per (128-row tile, head).  A chunk has an item
+        # for every head: with 128 heads even a single one fills the GPU, so its keys are never split
+        self.item_cap = chunks * heads
         self.items = torch.empty(self.item_cap * 8, dtype=torch.int32, device=device)
         self.n_items = torch.zeros(1, dtype=torch.int32, device=device)
-        self.row_ns = torch.zeros(max_rows, dtype=torch.int32, device=device)
-        self.opart = self.lse = None
+        self.row_ns = torch.zeros(max_rows, dtype=torch.int32, device=device)      # first word: the counter by which items are handed out
 
 
 def latent_gather(ws: PrefillWorkspace, cache, scale, page_table, spans, n_spans, max_tiles):
@@ -145,6 +142,6 @@ def prefill_attention(q, ws: PrefillWorkspace, n_tokens, seq, pos, softmax_scale
     T = q.shape[0]
     assert T <= ws.max_rows and n_tokens <= ws.budget
     native.call("plow_mla_prefill_attention", q, ws.kvb, ws.krope, int(n_tokens), ws.vpt, ws.vpt.shape[1], seq, pos, T, ws.heads,
-                ws.tiles_per_split, ws.max_splits, ws.items, ws.item_cap, ws.n_items, ws.row_ns, ws.opart, ws.lse, out,
+                ws.items, ws.item_cap, ws.n_items, ws.row_ns, out,
                 float(softmax_scale), native.status_word(q.device))
     return out

@@ -152,7 +152,7 @@ _SIGS = {
     "plow_sigmoid_gate": "ppplp",
     "plow_gqa_attention": "ppplpipp" "iiiiiii" "pi" "ppppp" "fpppp",
     "plow_rope_kv": "ppi" "pppppppp" "i" "iiiiiii" "fppp",
-    "plow_mla_prefill_attention": "ppplpipp" "iiii" "pi" "ppppp" "fpp",
+    "plow_mla_prefill_attention": "ppplpipp" "ii" "pi" "ppp" "fpp",
     "plow_mla_latent_gather": "ppipppppp" "ipiiiip",
     "plow_mla_q_rope": "pippiiiiip",
 }
