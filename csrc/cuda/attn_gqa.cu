@@ -950,7 +950,7 @@ int plow_rope_kv(void* q_out, const void* qkv, int ld_qkv, void* kc, void* vc, c
           page_table, max_pages, rows, nq, nkv, pair_mode, plus_one, eps, kv_scale);
     };
     // eight heads a warp once that leaves every SM a block
-    if (static_cast<long long>(rows) * heads >= 148 * 8 * 8) run(rope_kv128_kernel<8>, 8); else run(rope_kv128_kernel<1>, 1);
+    if (static_cast<long long>(rows) * heads >= sm_count() * 8 * 8) run(rope_kv128_kernel<8>, 8); else run(rope_kv128_kernel<1>, 1);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : 4000 + static_cast<int>(e);
   }

@@ -506,7 +506,7 @@ int plow_dsa_select(int* sel, float* scores, int ld_scores, void* q8, float* wq,
   // CTAs per row: while the rows alone leave SMs idle or a CTA would hold over a quarter of its room (two to four stay
   // resident per SM), but none with under 1024 elements, where the cluster's barriers cost more than the passes
   int nc = 1;
-  while (nc < kTopCluster && ((max_len + nc - 1) / nc > kTopSlice / 4 || static_cast<long long>(rows) * nc < 2 * 148) && max_len / (2 * nc) >= 1024) nc <<= 1;
+  while (nc < kTopCluster && ((max_len + nc - 1) / nc > kTopSlice / 4 || static_cast<long long>(rows) * nc < 2 * sm_count()) && max_len / (2 * nc) >= 1024) nc <<= 1;
   const int slice = ((max_len + nc - 1) / nc + 31) & ~31;
   const int slice_cap = slice <= kTopSlice ? slice : 0;
   static DeviceOnce attr2;

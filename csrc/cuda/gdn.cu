@@ -6,7 +6,7 @@
 //   S     <- alpha S;   S <- S + beta (v - S k) (x) k;   o = S q / sqrt(d)       S[V][K] f32 per (sequence, v head)
 //   out    = RMSNorm(o) * gamma * SiLU(z)                                  per (token, v head)
 //
-// A call is three kernels.  gdn_prep_kernel does what is independent per token: convolution, SiLU, the norms, the gates and
+// A call is two kernels, above kShortRows rows three.  gdn_prep_kernel does what is independent per token: convolution, SiLU, the norms, the gates and
 // the dot products of neighbouring tokens, into f32 scratch, and lists the runs (consecutive rows of one sequence).  The
 // recurrence walks the runs: gdn_long_kernel those of kLongRun rows and more, gdn_short_kernel the others (decode; up to
 // kShortRows rows take it alone).  Row i of S depends on the whole of k but on no other row, so a (run, v head) is cut into
@@ -25,6 +25,7 @@
 #include <stdint.h>
 
 #include "launch.cuh"
+#include "tmap.cuh"
 
 namespace {
 
@@ -765,9 +766,10 @@ int plow_gdn(void* out, float* conv_state, float* ssm_state, const void* qkvz, i
   static plow::DeviceOnce attr;
   if (rows > kShortRows && plow::ensure_smem(attr, gdn_long_kernel, kLongSmem) != cudaSuccess) return 3000;
   if (rows > kShortRows)
-    plow::launch_serial(gdn_long_kernel, dim3(148), dim3(kHalves * kRecurThreads), kLongSmem, cs, o, ssm_state, sc, pos, seq, rows, hk, hv, vec_s);
+    plow::launch_serial(gdn_long_kernel, dim3(plow::sm_count()), dim3(kHalves * kRecurThreads), kLongSmem, cs, o, ssm_state, sc, pos, seq, rows, hk, hv, vec_s);
   const long long most = static_cast<long long>(rows) * (hv * kSplit + ((2 * hk + hv) * kD + kConvItem - 1) / kConvItem);
-  const int grid = static_cast<int>(most < 148 * 4 ? most : 148 * 4);
+  const int room = 4 * plow::sm_count();
+  const int grid = static_cast<int>(most < room ? most : room);
   plow::launch_serial(gdn_short_kernel, dim3(grid), dim3(kRecurThreads), 0, cs, o, conv_state, ssm_state, sc, x, ld_qkvz, pos, seq, rows, hk, hv,
                       vec_s, rows > kShortRows ? 0 : 1);
   cudaError_t e = cudaGetLastError();
