@@ -17,7 +17,7 @@ class KernelSpec:
     dtypes: tuple             # operand dtypes accepted
     constraints: dict = field(default_factory=dict)   # attr -> allowed values / (lo, hi) range / callable
     uses: tuple = ()          # ISA features: tcgen05, tmem, tma, peer
-    smem_bytes: int = 0
+    smem_bytes: int = 0       # shared memory and TMEM: the most that any kernel behind the launcher takes
     tmem_cols: int = 0
     regs: int = 0             # filled from the ptxas report
     alias_group: str = ""     # kernels that may stand in for one another
@@ -28,18 +28,19 @@ REGISTRY = [
     KernelSpec("plow_gemm", "linear_glu", ("bf16", "e4m3"), dict(n_multiple=128), ("tcgen05", "tmem", "tma"), 203776, 512, alias_group="gemm"),
     KernelSpec("plow_gemm", "moe_experts", ("bf16", "e4m3"), dict(n_multiple=128), ("tcgen05", "tmem", "tma"), 203776, 512, alias_group="gemm"),
     KernelSpec("plow_gemm", "gemm_xreduce", ("bf16", "e4m3"), dict(rows=(1, 64), n_multiple=8), ("tcgen05", "tmem", "tma", "peer"), 203776, 512),
-    KernelSpec("plow_gqa_attention", "attention", ("bf16",), dict(head_dim=(128, 256), group_pow2=True), ("tcgen05", "tmem", "tma"), 198656, 256),
+    KernelSpec("plow_gqa_attention", "attention", ("bf16",), dict(head_dim=(128, 256), group_pow2=True), ("tcgen05", "tmem", "tma"), 211968, 512),
     KernelSpec("plow_rope_kv", "rope_kv", ("bf16",), dict(head_dim_multiple=8)),
     KernelSpec("plow_mla_decode", "mla_attention", ("e4m3",), dict(heads=(128,), kv_lora=(512,), qk_rope=(64,)), ("tcgen05", "tmem", "tma"), 203776, 512),
     KernelSpec("plow_mla_absorb", "mla_attention", ("bf16",), dict(qk_nope=(128,)), ("tcgen05", "tmem", "tma")),
     KernelSpec("plow_mla_fold", "mla_attention", ("bf16",), dict(v_head=(128,), max_splits=(1, 8)), ("tcgen05", "tmem", "tma")),
+    KernelSpec("plow_mla_prefill_attention", "mla_attention", ("bf16",), dict(qk_nope=(128,), qk_rope=(64,), v_head=(128,)), ("tcgen05", "tmem", "tma"), 219136, 512),
     KernelSpec("plow_mla_kv_write", "mla_kv_write", ("e4m3",)),
     KernelSpec("plow_dsa_k_write", "dsa_k_write", ("e4m3",), dict(dim=(128,))),
-    KernelSpec("plow_dsa_select", "dsa_topk", ("e4m3",), dict(heads=(64,), dim=(128,), max_len=(1, 1 << 20)), ("tcgen05", "tmem", "tma"), 75776, 128),
-    KernelSpec("plow_gdn", "gdn", ("bf16",), dict(head_dim=(128,), conv=(4,))),
+    KernelSpec("plow_dsa_select", "dsa_topk", ("e4m3",), dict(heads=(64,), dim=(128,), max_len=(1, 1 << 20)), ("tcgen05", "tmem", "tma"), 180416, 128),
+    KernelSpec("plow_gdn", "gdn", ("bf16",), dict(head_dim=(128,), conv=(4,)), (), 57216),
     KernelSpec("plow_gated_norm", "gated_norm", ("bf16",)),
     KernelSpec("plow_router_topk", "router_topk", ("f32",), dict(n_experts=(1, 1024))),
-    KernelSpec("plow_sample", "sample", ("f32",)),
+    KernelSpec("plow_sample", "sample", ("f32",), {}, (), 213328),
     KernelSpec("plow_rmsnorm", "rmsnorm", ("bf16",)),
     KernelSpec("plow_add_norm", "add_norm", ("bf16",)),
     KernelSpec("plow_interp_run", "row_segment", ("bf16",), dict(ops=("embed", "rmsnorm", "add_norm", "add", "silu_mul", "row_gather", "argmax"))),
