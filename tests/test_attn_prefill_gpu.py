@@ -189,11 +189,11 @@ def test_rope_kv_layouts(rows, nq, nkv, pair_mode, norm, kv8, pad):
     def cells(c, o):
         c = c[page, at]
         return c.view(torch.float8_e4m3fn).float() * ks[page, at][:, o:o + nkv, None] if kv8 else c.float()
-    # one bf16 rounding (of the norm too, which the rotation mixes between two values), or one e4m3 rounding of a 448-scaled row
-    tol = 2.0 ** -4 if kv8 else 2.0 ** -7
-    for got, want in ((q[live].float(), rot(x[:, :nq], qn)), (cells(kc, 0), want_k), (cells(vc, nkv), want_v)):
-        t = 2.0 ** -7 if got is not None and got.shape[1] == nq and not kv8 else tol
-        assert ((got - want).abs() <= t * want.abs().amax(-1, keepdim=True)).all()
+    # one bf16 rounding (of the norm too, which the rotation mixes between two values); cells of the e4m3 cache one rounding of a
+    # 448-scaled row
+    cell = 2.0 ** -4 if kv8 else 2.0 ** -7
+    for got, want, tol in ((q[live].float(), rot(x[:, :nq], qn), 2.0 ** -7), (cells(kc, 0), want_k, cell), (cells(vc, nkv), want_v, cell)):
+        assert ((got - want).abs() <= tol * want.abs().amax(-1, keepdim=True)).all()
     assert (q[pos < 0] == 7.0).all()
 
 

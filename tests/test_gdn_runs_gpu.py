@@ -34,7 +34,9 @@ def _case(lens, starts, hk, hv, idle, pad, seed):
 @pytest.mark.parametrize("lens,starts,hk,hv,idle,pad", [
     ([1], [0], 2, 4, 0, 0), ([1, 1, 1], [0, 5, 9], 16, 32, 1, 0), ([2, 3, 4], [0, 7, 0], 2, 2, 0, 0),
     ([7, 8, 9, 1, 2], [0, 11, 0, 3, 1], 2, 4, 2, 1), ([15, 16, 17, 18], [4, 0, 1, 2], 1, 4, 0, 3),
-    ([100, 1, 301], [0, 64, 1000], 2, 4, 1, 2), ([70, 5, 4, 3, 66], [0, 1, 0, 9, 2], 2, 4, 1, 0), ([25, 24, 23, 1, 1, 1, 200], [0, 1, 2, 3, 4, 5, 6], 2, 4, 0, 4)])
+    ([100, 1, 301], [0, 64, 1000], 2, 4, 1, 2), ([70, 5, 4, 3, 66], [0, 1, 0, 9, 2], 2, 4, 1, 0), ([25, 24, 23, 1, 1, 1, 200], [0, 1, 2, 3, 4, 5, 6], 2, 4, 0, 4),
+    # 128 items a run: more than blocks (the second halves take some), more than halves (a half takes several, short runs skipped between)
+    ([41, 50], [3, 0], 16, 32, 0, 0), ([3, 40, 1, 2, 27, 4, 9], [0, 5, 9, 0, 2, 7, 1], 16, 32, 1, 0), ([1] * 40, list(range(40)), 16, 32, 0, 0)])
 def test_gdn_runs(lens, starts, hk, hv, idle, pad):
     from plow_b200.ops import gdn
     qkvz, ba, conv_w, a_log, dt_bias, cs, ss, pos, seq, spans = _case(lens, starts, hk, hv, idle, pad, sum(lens))
