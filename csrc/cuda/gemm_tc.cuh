@@ -252,7 +252,9 @@ struct TileSched {
 // silu with the approximate reciprocal (2 ulp): the exact division cost the epilogue warps ~350 clocks per value
 __device__ __forceinline__ float silu_f(float v) { return __fdividef(v, 1.0f + __expf(-v)); }
 
-// acc += v * f for two neighbouring accumulators: one packed instruction (the promotion is bound by issue)
+// acc += v * f for two neighbouring accumulators: one packed instruction.  The promotion is bound by the exposed wait for its TMEM reads and
+// only in part by issue, so the packed form pays where the epilogue also holds the gate and up halves (2048 x 2 x 18432 x 7168: 524 us,
+// 544 with two scalar instructions); without those the scalar ones are faster (2048 x 7168 x 18432: 415 us, 451 packed).
 __device__ __forceinline__ void fma_pair(float& a0, float& a1, uint32_t v0, uint32_t v1, float f0, float f1) {
   asm("{\n\t.reg .b64 a, v, f;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tmov.b64 f, {%4, %5};\n\t"
       "fma.rn.f32x2 a, v, f, a;\n\tmov.b64 {%0, %1}, a;\n\t}\n"
@@ -547,8 +549,15 @@ gemm_tc_kernel(const GemmArgs a, const __grid_constant__ CUtensorMap tm_x,
                     const float fs = s0.sa[0] * ((DUAL && col >= kCH) ? s0.wu : s0.wg);
                     f = make_float4(fs, fs, fs, fs);
                   }
-                  fma_pair(acc[col], acc[col + 1], v[q * 16 + j], v[q * 16 + j + 1], f.x, f.y);
-                  fma_pair(acc[col + 2], acc[col + 3], v[q * 16 + j + 2], v[q * 16 + j + 3], f.z, f.w);
+                  if constexpr (DUAL) {
+                    fma_pair(acc[col], acc[col + 1], v[q * 16 + j], v[q * 16 + j + 1], f.x, f.y);
+                    fma_pair(acc[col + 2], acc[col + 3], v[q * 16 + j + 2], v[q * 16 + j + 3], f.z, f.w);
+                  } else {
+                    acc[col] = fmaf(__uint_as_float(v[q * 16 + j]), f.x, acc[col]);
+                    acc[col + 1] = fmaf(__uint_as_float(v[q * 16 + j + 1]), f.y, acc[col + 1]);
+                    acc[col + 2] = fmaf(__uint_as_float(v[q * 16 + j + 2]), f.z, acc[col + 2]);
+                    acc[col + 3] = fmaf(__uint_as_float(v[q * 16 + j + 3]), f.w, acc[col + 3]);
+                  }
                 }
               }
             }
