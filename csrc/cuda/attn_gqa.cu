@@ -1,5 +1,7 @@
-// Grouped-query flash attention over a paged bf16 KV cache, on tcgen05 — one kernel for prefill and
-// decode — plus the fused head-norm + RoPE + cache-write row op that feeds it.
+// Grouped-query flash attention over a paged KV cache: the launcher, the one-tile kernel on tcgen05, and the fused head-norm +
+// RoPE + cache-write row op that feeds it.  At head dim 128, decode steps of up to 256 rows (every row a sequence of its own) run
+// the streaming body of attn_decode.cuh, and bf16 calls of more than kPrefillRows rows whose keys are not split run
+// attn_prefill.cu; mixed and short calls, split keys, head dim 256 and runs over the e4m3 cache take the one-tile kernel.
 //
 // The step's query rows arrive as q[row][head][HD]; each row carries (slot, position) and attends
 // to the cached positions t <= position of its slot (optionally t > position - window), which makes
@@ -24,7 +26,7 @@
 //
 // e4m3 cache (KV8 instantiation): K and V cells are e4m3 bytes with one f32 scale per (token, kv head).  The TMA warp
 // brings the raw byte tiles into a staging ring; converter warps rewrite each tile as bf16 operands in the layout the
-// MMAs read (the 128-byte swizzle a bf16 TMA load would produce) and hand the stage to the MMA warp.  The rewrite is
+// MMAs read (the 128-byte swizzle a bf16 TMA load would produce) and hand the stage to the MMA warp.
 // The rewrite is three integer instructions per element pair: the e4m3 byte s.eeee.mmm placed as the bf16
 // s.0000eeee.mmm0000 is exactly value * 2^-120 (normal and subnormal codes alike), so no float conversion is needed;
 // the per-token scales and the 2^120 go where a multiplication already is or costs one instruction: S columns are
@@ -46,8 +48,11 @@ constexpr int kGqaThreads = 192;   // TMA warp, MMA warp, 4 softmax warps
 constexpr int kGqaThreads8 = 320;  // + 4 converter warps (e4m3 cache)
 constexpr int kGqaRaw = 3;         // raw e4m3 tiles in flight; 4 operand stages behind them
 
-// Rows from which an unsplit bf16 call takes the two-tile kernel of attn_prefill.cu: its items are up to twice as long, so
-// it wants many rows; decode steps (one row per sequence) lie below.
+// Rows above which a bf16 call that does not split its keys takes the two-tile kernel of attn_prefill.cu, which cannot split them;
+// decode steps (one row per sequence) lie below.  A workspace that chooses its own splits leaves keys whole once its rows make
+// two one-tile items per SM (32 / 8 heads: from 1153 rows on), so between here and there the split one-tile kernel runs.  Unsplit, the
+// two-tile kernel is the faster one over that range as well (512 rows 26.5 us against 54.2, behind 4096 85.6 / 107.5; 257 rows behind
+// 4096 80.9 / 82.6): the line follows the workspace's split count and not these figures.
 constexpr int kPrefillRows = 256;
 
 struct GqaItem { int r0, nt, kvh, split, tile0, ntiles, slot, ns; };

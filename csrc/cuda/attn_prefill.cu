@@ -14,12 +14,13 @@
 //
 // Items are (chunk of up to two tiles of consecutive rows, kv head); chunks are sorted by length on the device, items
 // handed out through a counter, longest first, so the last ones are short.  With many heads they come in groups of as many
-// heads as give every SM two items: the heads at work then share their keys in L2 (128 heads of 4096 tokens are 268 MB).  Masks, lazy rescaling and numerics are those of attn_gqa.cu.
+// heads as give every SM two items: the heads at work then share their keys in L2 (128 heads of 4096 tokens are 268 MB).  Masks, lazy rescaling
+// and numerics are those of attn_gqa.cu.
 //
-// 4096 tokens, 32 / 8 heads: 154 us with the chunk list, the one-tile kernel with its list took 248 (892 against 554
-// TFLOP/s); latent attention, 2048 rows behind 2048, 128 heads: 520 us against 632.  What bounds it: the chain of one tile
-// (S ready, maximum, exponentials, P, P V, Q K^T, about 3000 clocks) is longer than the 2048 tensor clocks of the two tiles,
-// so the tensor pipe is busy two thirds of the time.  Tried and worse: an MMA warp per tile (166), waiting for the slabs
+// 4096 tokens, 32 / 8 heads: 154 to 158 us with the chunk list, the one-tile kernel with its list took 248 (890 to 868 against 554
+// TFLOP/s); latent attention, 2048 rows behind 2048, 128 heads: 515 us against 632.  What bounds it: the chain of one tile
+// (S ready, maximum, exponentials, P, P V, Q K^T, about 3000 clocks) is longer than the 2048 tensor clocks of the two tiles.
+// Over a whole launch the tensor pipe is active 45 % (latent: 50 %) of the time, issue slots 46 %, the exponentials' pipe 36 %.  Tried and worse: an MMA warp per tile (166), waiting for the slabs
 // before P instead of after (165).
 #include <cuda_bf16.h>
 

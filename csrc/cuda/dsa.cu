@@ -11,7 +11,8 @@
 // the row's 64 index heads the B operand (N = 64), K = 128 e4m3: D[token][head] lands with one token
 // per TMEM lane, so the weighted ReLU sum over heads is a private 64-column loop per thread and the
 // score leaves the kernel with one coalesced store.  One warp keeps a ring of four tiles and two accumulators busy,
-// four warps read them back; three CTAs per SM.  It is bound by the stream of the index keys.  (A CTA per tile paid
+// four warps read them back; three CTAs per SM.  DRAM is half busy while it runs; the warps wait for the keys' scales and
+// the read-back.  (A CTA per tile paid
 // barrier and TMEM set-up and one exposed TMA -> MMA -> read-back chain for every 16 KB: 106 us for 64 rows x 32768,
 // 68 us now.)
 //
@@ -19,7 +20,7 @@
 // of the key range finds the bin that holds the cut; its elements (a few hundred) are sorted by the first CTA, which gives
 // the cut value and how many of its ties are taken, lowest index first; a last pass writes the selection in index order.
 // (One CTA per row took seven 8-bit digit passes over
-// global memory: 121 us for 64 rows x 32768, top 2048; 65 us now.)
+// global memory: 121 us for 64 rows x 32768, top 2048; 51 to 65 us now, half of the stalls at the barriers of CTAs and clusters.)
 #include <cuda_bf16.h>
 #include <cooperative_groups.h>
 #include <cuda_fp8.h>

@@ -6,8 +6,8 @@
 //   S     <- alpha S;   S <- S + beta (v - S k) (x) k;   o = S q / sqrt(d)       S[V][K] f32 per (sequence, v head)
 //   out    = RMSNorm(o) * gamma * SiLU(z)                                  per (token, v head)
 //
-// A call is two kernels, above kShortRows rows three.  gdn_prep_kernel does what is independent per token: convolution, SiLU, the norms, the gates and
-// the dot products of neighbouring tokens, into f32 scratch, and lists the runs (consecutive rows of one sequence).  The
+// A call is two kernels, above kShortRows rows three.  gdn_prep_kernel does what is independent per token: convolution, SiLU,
+// the norms, the gates and the dot products of neighbouring tokens, into f32 scratch, and lists the runs (consecutive rows of one sequence).  The
 // recurrence walks the runs: gdn_long_kernel those of kLongRun rows and more, gdn_short_kernel the others (decode; up to
 // kShortRows rows take it alone).  Row i of S depends on the whole of k but on no other row, so a (run, v head) is cut into
 // four items of 32 rows and one prompt fills 128 SMs with hv = 32; inside a CTA eight lanes share a pair of rows (16 of the
@@ -17,7 +17,7 @@
 //     o_i = c_i R_i + sum_{j<=i} (a_{j+1} .. a_i) d_j (k_j . q_i),  S  <- c_n S + sum_j (a_{j+1} .. a_n) d_j k_j
 // which is the recurrence above with its sums regrouped, all in f32.  What bounds it is the issue of the packed FMAs and
 // the shared-memory reads of k and q (every thread reads its 16 columns), and between them the serial part of a step: one
-// warp per scheduler, 565 instructions and 1780 clocks for four tokens.  2048 tokens of one prompt, 32 heads: 530 us, of
+// warp per scheduler, 565 instructions and 1780 clocks for four tokens (issue slots 33 % busy, the stalls are fixed latencies).  2048 tokens of one prompt, 32 heads: 530 us, of
 // which 460 the recurrence (two tokens a step: 725) and 55 the preparation; 64 decode rows 67 us.  One CTA per (run, head)
 // that also convolved, with 128 columns per thread and two block reductions a token, took 4880 us and 191 us.
 #include <cuda_bf16.h>
@@ -95,7 +95,8 @@ __device__ __forceinline__ void unpack4(uint2 u, float* x) {
 
 // One warp per (RB rows, head slot): slots [0, hk) are the q and k channels of a key head, [hk, hk + hv) the v channels of a
 // v head; a lane owns four consecutive channels and keeps its taps and the last three keys in registers while it walks the
-// rows, the next row's inputs already requested.  What bounds it is instruction issue (about 300 per row of a key head), so
+// rows, the next row's inputs already requested.  What bounds it is instruction issue (about 300 per row of a key head, slots 53 % busy with the 15
+// warps an SM that 126 registers leave), so
 // the walk is a loop: unrolled over its rows, with every row's inputs up front, it took 80 us for 2048 rows and spent a
 // quarter of the time fetching instructions.  The first block column lists the runs.
 template <int RB>

@@ -8,8 +8,9 @@
 // logits in shared memory and all later passes run there, partial results crossing the cluster through distributed
 // shared memory.  (One 1024-thread CTA per row that re-read the row for each of up to twelve passes and counted into one
 // shared histogram with atomics took 2620 us for 256 rows x 128256: the leading digit of the logits hits a handful of
-// counters, and shared f32 atomics are compare-and-swap loops.  This kernel: 210 us, 10 us for one unfiltered row.  It is
-// bound by instruction issue of the passes, not by memory: reading the logits alone takes 20 us.)
+// counters, and shared f32 atomics are compare-and-swap loops.  This kernel: 213 us, 15 to 19 us for one
+// unfiltered row of 32000 or 128256.  It is bound by the chain of passes, not by memory: reading the logits alone takes 20 us, DRAM is
+// 6 % and issue slots are 43 % busy, and the longest stalls are at the barriers of the CTAs and clusters.)
 //
 // The cut of a filter - the largest key T such that weight({key >= T}) >= target, weight = element count for top-k,
 // probability mass for top-p - is found by narrowing: 16 bins of the distance to the maximum (later: of the key range of
@@ -433,7 +434,8 @@ sample_kernel(int* out, const float* logits, int ld, int V, int slice, int in_sm
   if (T <= 0.f) {
     if (greedy_alone) {
       // The CTAs do not fit the chip at once: a greedy row, which reads its logits once, gives its cluster's places back (128 rows x
-      // 128256, all greedy: 36 us, 44 with the whole cluster at work; with all resident one row of 128256 takes 13 us, alone 25).
+      // 128256, all greedy: 36 us, 44 with the whole cluster at work; 64 rows 26 either way.  Where all are resident the cluster is
+      // the faster one: one row of 128256 13 us).
       if (r.rank) return;
       r.n = V; r.nc = 1;
     }

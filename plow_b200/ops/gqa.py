@@ -2,9 +2,9 @@
 (csrc/cuda/attn_gqa.cu).
 
 ``rope_kv`` is the fused head-norm + RoPE + cache-write row op (reference op HEADNORM_ROPE,
-runtime/common/dev_isa.h:74-84); ``attention`` is the tcgen05 flash kernel that serves prefill
-(causal by position) and decode (one row per sequence) from the same work list
-(runtime/common/dev_isa.h:185-222).
+runtime/common/dev_isa.h:74-84); ``attention`` serves prefill (causal by position) and decode (one row per
+sequence) by the same rule (runtime/common/dev_isa.h:185-222), through the kernel that its rows and workspace call for:
+streaming decode, two-tile prefill or the one-tile kernel.
 """
 from __future__ import annotations
 

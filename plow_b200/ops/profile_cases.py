@@ -18,6 +18,8 @@ Cases
     gqa_prefill      one 4096-token prompt, 32/8 heads, hd128
     gqa_prefill_e4m3 the same over an e4m3 cache
     dsa_topk         64 rows x 32768 scores, exact top-2048
+    gdn_prefill      one run of 2048 tokens through the gated delta rule, 16 key / 32 value heads
+    sample           256 rows x 128256 logits, temperature 0.8, top-k 50 on half of them, top-p 0.9
 """
 from __future__ import annotations
 
@@ -188,6 +190,31 @@ def case_gqa_prefill(iters):
 def case_dsa_topk(iters):
     from . import dsa
     return dsa.profile_topk(iters, _time)
+
+
+def case_gdn_prefill(iters):
+    from . import gdn
+    T, hk, hv, d = 2048, 16, 32, 128
+    C = (2 * hk + hv) * d
+    qkvz = torch.randn(T, C + hv * d, device="cuda").bfloat16()
+    ba = torch.randn(T, 2 * hv, device="cuda").bfloat16()
+    conv_w, a_log, dt = torch.randn(C, 4, device="cuda") * 0.4, torch.rand(hv, device="cuda"), torch.randn(hv, device="cuda") - 4.0
+    cs, ss = torch.zeros(1, C, 3, device="cuda"), torch.zeros(1, hv, d, d, device="cuda")
+    pos, seq = torch.arange(T, dtype=torch.int32, device="cuda"), torch.zeros(T, dtype=torch.int32, device="cuda")
+    out = torch.empty(T, hv * d, dtype=torch.bfloat16, device="cuda")
+    us = _time(lambda: gdn.gdn(qkvz, ba, conv_w, a_log, dt, cs, ss, pos, seq, hk, hv, out=out), iters)
+    return dict(us=us, flops=6.0 * T * hv * d * d, bytes=2.0 * T * (C + hv * d) + 4.0 * hv * d * d)
+
+
+def case_sample(iters):
+    from . import sampler
+    R, V = 256, 128256
+    logits = torch.randn(R, V, device="cuda") * 2.5
+    half = torch.arange(R, device="cuda") % 2
+    t, k, p, m = torch.full((R,), 0.8, device="cuda"), (half * 50).int(), torch.full((R,), 0.9, device="cuda"), torch.zeros(R, device="cuda")
+    u = torch.rand(R, device="cuda")
+    us = _time(lambda: sampler.sample(logits, t, k, p, m, u=u), iters)
+    return dict(us=us, flops=4.0 * R * V, bytes=4.0 * R * V)
 
 
 CASES = {k[5:]: v for k, v in list(globals().items()) if k.startswith("case_")}
