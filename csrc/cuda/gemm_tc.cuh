@@ -255,7 +255,8 @@ __device__ __forceinline__ float silu_f(float v) { return __fdividef(v, 1.0f + _
 // acc += v * f for two neighbouring accumulators: one packed instruction.  The promotion is bound by the exposed wait for its TMEM reads and
 // only in part by issue, so the packed form pays where the epilogue also holds the gate and up halves (2048 x 2 x 18432 x 7168: 524 us,
 // 544 with two scalar instructions); without those the scalar ones are faster where K is long (2048 x 7168 x 18432: 415 us, 451 packed)
-// and a little slower where it is short (4096 x 32768 x 512: 184 us, 179 packed).
+// and slower where it is short or the weights lie in L2 (4096 x 32768 x 512: 184 us, 179 packed; weights in L2, 2048 x 7168 x 2048
+// 48.2 / 46.2, x 7168 131.5 / 125, x 16384 410 / 440).
 __device__ __forceinline__ void fma_pair(float& a0, float& a1, uint32_t v0, uint32_t v1, float f0, float f1) {
   asm("{\n\t.reg .b64 a, v, f;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 v, {%2, %3};\n\tmov.b64 f, {%4, %5};\n\t"
       "fma.rn.f32x2 a, v, f, a;\n\tmov.b64 {%0, %1}, a;\n\t}\n"
